@@ -136,7 +136,13 @@ typedef struct {
                             (0x10000) turns them off; bits 8..15: B rows
                             the staged walk loads ahead (0 = 4); bits
                             20..27: rows a row group takes in a run (0 =
-                            16, shorter for small bins)                    */
+                            16, shorter for small bins).
+                            0 also computes rows that repeat one pattern
+                            at a fixed distance (structured grids and the
+                            products of their aggregations) in runs, with
+                            no hashing per row, when the product is large
+                            enough to pay for the search; 8 = 0 with runs
+                            at any size; bit 16 turns them off              */
   int32_t sym_fill_pct;  /* symbolic bin thresholds: a row goes to the bin
                             whose table (32 << b slots) it fills to at most
                             this percentage at its upper bound of distinct
@@ -248,7 +254,7 @@ int nspb_spgemm_host(const nspb_csr_in *hA, const nspb_csr_in *hB, int32_t *h_ro
 /* ---- autotuner ---------------------------------------------------------------
  * Times this product (C sized once, then written into the same arrays) under
  * candidates of the row-group threads per row (group_lanes 8, 16, 32), kernel
- * family (row_kernel 1 hash-sort, 2 staged walk), table size (num_table_shift
+ * family (row_kernel 1 hash-sort, 2 staged walk, 7 entry maps, 0), table size (num_table_shift
  * 0/1, or row_kernel 2/3) and bin thresholds (sym_fill_pct 50/75/90,
  * num_fill_pct 25/37/50), each knob swept in turn with the best values found
  * so far for the others: one warm-up and `reps` timed calls per candidate,

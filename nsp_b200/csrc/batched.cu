@@ -70,16 +70,16 @@ using namespace nspb;
 
 // Host-side description of one group's product table and the offsets of one
 // device block holding it: the per-product operands, each product's first
-// global row, the product of every global row, the group's row pointer and
-// the per-product starts in C.
+// global row, the product of every global row, the group's row pointer, the
+// per-product starts in C and the column shifts of every B's rows.
 struct TableHost {
   int count = 0;
   bool f32 = false;
-  long long rows = 0, a_nnz = 0, max_rows = 0;
+  long long rows = 0, a_nnz = 0, b_nnz = 0, brows = 0, max_rows = 0;
   int max_ncols = 0, max_brows = 0;
   std::vector<Operands<double>> ops;  // value pointers of fp32 operands stored as-is
   std::vector<int> row_off;
-  size_t o_ops = 0, o_roff = 0, o_por = 0, o_crp = 0, o_st = 0, bytes = 0;
+  size_t o_ops = 0, o_roff = 0, o_por = 0, o_crp = 0, o_st = 0, o_del = 0, bytes = 0;
 };
 
 static int table_layout(int count, const nspb_csr_in *A, const nspb_csr_in *B, bool f32,
@@ -111,6 +111,8 @@ static int table_layout(int count, const nspb_csr_in *A, const nspb_csr_in *B, b
     h.row_off[p] = (int)h.rows;
     h.rows += a.nrows;
     h.a_nnz += a.nnz;
+    h.b_nnz += b.nnz;
+    h.brows += b.nrows;
     h.max_rows = std::max<long long>(h.max_rows, a.nrows);
     h.max_ncols = std::max(h.max_ncols, b.ncols);
     h.max_brows = std::max(h.max_brows, b.nrows);
@@ -124,15 +126,21 @@ static int table_layout(int count, const nspb_csr_in *A, const nspb_csr_in *B, b
   h.o_por = off; off = al(off + 4 * (size_t)std::max<long long>(h.rows, 1));
   h.o_crp = off; off = al(off + 4 * (size_t)(h.rows + 1));
   h.o_st = off; off = al(off + 4 * (size_t)(count + 1));
+  h.o_del = off; off = al(off + sizeof(int2) * (size_t)kMaxLag * (size_t)h.brows);
   h.bytes = off;
   return NSPB_OK;
 }
 
 // Descriptors and row offsets to the device (`host` keeps the staging bytes
 // alive until the copy has run), then the row-to-product map.
-static cudaError_t table_build(const TableHost &h, char *ws, std::vector<char> &host,
+static cudaError_t table_build(TableHost &h, char *ws, std::vector<char> &host,
                                cudaStream_t s) {
   host.assign(h.o_por, 0);
+  int2 *del = reinterpret_cast<int2 *>(ws + h.o_del);  // each product's B row shifts
+  for (auto &o : h.ops) {
+    o.bdel = del;
+    del += (size_t)kMaxLag * o.brows;
+  }
   std::memcpy(host.data() + h.o_ops, h.ops.data(), sizeof(Operands<double>) * h.count);
   std::memcpy(host.data() + h.o_roff, h.row_off.data(), 4 * (size_t)(h.count + 1));
   cudaError_t e = cudaMemcpyAsync(ws, host.data(), h.o_por, cudaMemcpyHostToDevice, s);
@@ -158,7 +166,10 @@ static void table_of(const TableHost &h, char *ws, Call &call) {
   info.max_ncols = h.max_ncols;
   info.nprod = h.count;
   info.max_brows = h.max_brows;
+  info.brows = h.brows;
+  info.bdel = true;
   call.set_table(d, f, info, h.a_nnz);
+  call.b_nnz = h.b_nnz;
 }
 
 static void table_split(const TableHost &h, char *ws, int *rp_all, cudaStream_t s) {

@@ -420,6 +420,79 @@ __device__ __forceinline__ int bucket_of(int key, int lo, float scale, int nb) {
   return b < nb - 1 ? b : nb - 1;
 }
 
+// ---- tiles of consecutive rows --------------------------------------------------
+// The kernels that walk every row once (k_rowinfo, k_brow_delta) take a tile
+// of up to 256 rows a block, a thread a row, with the tile's columns staged in
+// shared memory by one coalesced read. Threads then walk their rows at the row
+// length's stride: odd lengths spread over the banks as they are; for even ones
+// (by the tile's middle row) entry e is kept at e + e/32.
+constexpr int kTileThreads = 256;
+constexpr int kTileCols = 8192;  // staged columns: 33 KB
+constexpr int kTileWords = kTileCols + kTileCols / 32;
+__device__ __forceinline__ int tile_at(int e, int skew) { return e + (e >> skew); }
+__device__ __forceinline__ int tile_skew(int len) { return len & 1 ? 31 : 5; }
+// Stages cols[e0, e1) (at most kTileCols): a thread has eight loads in flight,
+// 16 bytes each where the columns' alignment allows.
+__device__ __forceinline__ void tile_stage(const int *__restrict__ col, int e0, int e1, int skew,
+                                           int *__restrict__ words) {
+  const int n = e1 - e0;
+  const int *src = col + e0;
+  const int head = min(n, (int)((4u - (unsigned)(reinterpret_cast<size_t>(src) >> 2)) & 3u));
+  const int quads = (n - head) >> 2;
+  if ((int)threadIdx.x < head) words[tile_at(threadIdx.x, skew)] = __ldg(src + threadIdx.x);
+  const int rest = head + 4 * quads + (int)threadIdx.x;
+  if (rest < n) words[tile_at(rest, skew)] = __ldg(src + rest);
+  const int4 *q4 = reinterpret_cast<const int4 *>(src + head);
+  constexpr int kPer = kTileCols / 4 / kTileThreads;  // 8
+  int4 v[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int at = (int)threadIdx.x + i * kTileThreads;
+    if (at < quads) v[i] = __ldg(q4 + at);
+  }
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int at = (int)threadIdx.x + i * kTileThreads;
+    if (at < quads) {
+      const int e = head + 4 * at;
+      words[tile_at(e, skew)] = v[i].x;
+      words[tile_at(e + 1, skew)] = v[i].y;
+      words[tile_at(e + 2, skew)] = v[i].z;
+      words[tile_at(e + 3, skew)] = v[i].w;
+    }
+  }
+}
+// Column of entry e of a tile, by where the tile is: as staged, or in global
+// memory when it did not fit. `body` is instantiated for each, so that its
+// loops hold one kind of load.
+struct ColFlat {
+  const int *w;
+  int e0;
+  __device__ __forceinline__ int operator()(int e) const { return w[e - e0]; }
+};
+struct ColSkewed {
+  const int *w;
+  int e0;
+  __device__ __forceinline__ int operator()(int e) const { return w[tile_at(e - e0, 5)]; }
+};
+struct ColGlobal {
+  const int *p;
+  __device__ __forceinline__ int operator()(int e) const { return __ldg(p + e); }
+};
+template <typename F>
+__device__ __forceinline__ void with_cols(bool staged, int skew, const int *words, int e0,
+                                          const int *col, F &&body) {
+  if (!staged) body(ColGlobal{col});
+  else if (skew == 5) body(ColSkewed{words, e0});
+  else body(ColFlat{words, e0});
+}
+// Rows of a tile so that most tiles of a matrix of this mean row fit.
+inline int tile_rows(double mean) {
+  int r = kTileThreads;
+  while (r > 32 && r * mean > 0.9 * kTileCols) r >>= 1;
+  return r;
+}
+
 // True when B rows k and kt are one run of shifted rows (bit k of bits: B row k is row k-1 moved by one
 // column shift; launch_brow_shift);
 // runs are only followed over 31 rows at most (false beyond).

@@ -41,6 +41,7 @@ struct Operands {
   const VT *bval = nullptr;
   int ncols = 0;  // columns of B
   int brows = 0;  // rows of B
+  int2 *bdel = nullptr;  // B's row shifts and lengths (launch_brow_delta), or none
 };
 
 // The products a call computes, as the row kernels see them. A call's rows
@@ -67,6 +68,7 @@ inline ProdTable<void> structure_of(const ProdTable<VT> &t) {
   s.one.bval = t.one.bval;
   s.one.ncols = t.one.ncols;
   s.one.brows = t.one.brows;
+  s.one.bdel = t.one.bdel;
   s.ops = reinterpret_cast<const Operands<void> *>(t.ops);
   s.prod_of_row = t.prod_of_row;
   s.row_off = t.row_off;
@@ -81,6 +83,8 @@ struct ProdInfo {
   int max_ncols = 0;
   int nprod = 1;
   int max_brows = 0;
+  long long brows = 0;  // rows of every product's B
+  bool bdel = false;    // a table whose products have room for their B row shifts
 };
 
 // Inclusive row limits of the symbolic and numeric bins (the last bin of each
@@ -125,6 +129,37 @@ struct MapArgs {
 constexpr int kTemplateRun = 16;
 constexpr int kNoRowTemplates = 0x10000;
 
+// ---- row runs (rowrun.cu) ---------------------------------------------------------
+// Column shift of a B row against the row 1, 2 or 3 before it: kNoShift when
+// it is not that row moved by one shift, kAnyShift when both are empty.
+constexpr int kMaxLag = 3;
+constexpr int kNoShift = (int)0x80000000;
+constexpr int kAnyShift = 0x7fffffff;
+constexpr int kShiftMaxLen = 128;  // longer B rows are not compared
+constexpr int kRunMaxA = 128;      // A entries of a row in a run
+constexpr int kRunMaxIp = 1536;    // products of a row in a run
+constexpr int kRunMin = 6;         // rows of the shortest run
+// A run: rows row0, row0 + s, ..., `len` of them; meta = s | sigma << 2 | len << 4.
+struct RowRun {
+  int row0;
+  int meta;
+  int prog;  // its pattern's slot, then its program
+  int pad;
+};
+inline long long run_capacity(long long n) { return n / kRunMin + 1; }
+// The patterns of the runs: a table of representatives (run index + 1, 0:
+// free), the program of each slot and the representative run of each program.
+constexpr int kRunSlots = 1024;
+struct RunHead {
+  int nfound;    // runs found
+  int nprog;     // patterns among them
+  int nruns[2];  // runs kept: of few, of many products a row
+};
+struct RunTable {
+  RunHead *head = nullptr;
+  int *rep = nullptr, *prog_of = nullptr, *run_of = nullptr;  // kRunSlots each; rep zeroed
+};
+
 // fp32 input modes (compensated pairs, or fp64 accumulation of exact products).
 inline bool fp32_inputs(int precision) {
   return precision == NSPB_PREC_FP32_COMP || precision == NSPB_PREC_FP32_WIDE;
@@ -139,6 +174,15 @@ struct CompArgs {
 };
 
 // ---- rowinfo.cu -----------------------------------------------------------------
+// What launch_rowinfo needs to find rows that repeat an earlier row's pattern
+// (codes null: not wanted).
+struct RunScan {
+  unsigned char *codes = nullptr;  // per row: s | sigma << 2, or 0
+  const int *lag_count = nullptr;  // B rows with a shift at lag 1, 2, 3 (at [1..3])
+  long long brows = 0;             // rows of B: a lag counts from two fifths of them
+  bool codes_only = false;         // nothing else is wanted: skip all when no lag counts
+  bool same = false;               // A is B: its rows' links are B's shifts
+};
 cudaError_t launch_check_sorted(const CsrDev &B, int *flags, cudaStream_t s);
 // The B rows of every product of a table (ops: device array of nprod entries).
 cudaError_t launch_check_sorted_table(const Operands<void> *ops, int nprod, int max_brows,
@@ -154,14 +198,16 @@ cudaError_t launch_rowinfo(const ProdTable<void> &t, int n, int64_t a_nnz, const
                            int *row_nz,
                            int64_t *row_ip, int *sym_counts,
                            unsigned long long *total_ip, int *flags, int *long_list,
-                           int *long_count, cudaStream_t s);
+                           int *long_count, const RunScan &runs, cudaStream_t s);
 // Scatter rows into bin-contiguous order. kind 0: key = ub (symbolic bins),
 // kind 1: key = crpt[i+1]-crpt[i] (numeric bins). offsets: 16 bin starts.
 struct BinOffsets {
   int v[16];
 };
+// member (may be null): rows with a non-zero byte belong to a run and are left out.
 cudaError_t launch_perm(const int *key, int n, int kind, BinOffsets offsets,
-                        const BinLimits &lim, int *cursor, int *perm, cudaStream_t s);
+                        const BinLimits &lim, const unsigned char *member, int *cursor, int *perm,
+                        cudaStream_t s);
 // Reorder row lists of perm (list i: perm[off[i] .. off[i]+count[i])) so that
 // rows of the heaviest weight class come first; weight as in launch_perm.
 // Lists of more than kOrderCap rows are left as they are.
@@ -199,6 +245,8 @@ cudaError_t launch_symbolic_bin(int bin, int lanes, bool b_sorted, const ProdTab
 // column shift (same length, same column differences).
 cudaError_t launch_brow_shift(const int *brpt, const int *bcol, int nb, unsigned *bits,
                               cudaStream_t s);
+// The same bits from the shifts of launch_brow_delta.
+cudaError_t launch_shift_bits(const int2 *bdel, int nb, unsigned *bits, cudaStream_t s);
 cudaError_t launch_symbolic_map(int bin, int lanes, const ProdTable<void> &t, const int *rows,
                                 int count, int *row_nz, int *err, const MapArgs &m,
                                 cudaStream_t s);
@@ -260,4 +308,34 @@ cudaError_t launch_numeric_comp_map(int bin, int lanes, const ProdTable<float> &
                                     const int *crpt, int *ccol, double *cval, const int *rows,
                                     int count, bool prefetch_a, int run, const unsigned *bshift, int nmax, int *redo,
                                     int *max_deg, int *err, cudaStream_t s);
+
+// ---- rowrun.cu ------------------------------------------------------------------
+// Column shifts of B's rows and their lengths into bdel (3 * nb: lag 1, 2, 3), the number of
+// shifts found per lag into lag_count[1..3], and (flags not null) B_UNSORTED.
+cudaError_t launch_brow_delta(const ProdTable<void> &t, const ProdInfo &info, int64_t b_nnz,
+                              int *lag_count, int *flags, cudaStream_t s);
+// The runs of launch_rowinfo's codes (found: run_capacity(n) entries), their
+// patterns and the list of those kept (runs: small ones from the front, large
+// ones from the back); codes[] becomes the members' flags, row_nz of every
+// member is zeroed and its symbolic bin counted in sym_sub.
+cudaError_t launch_run_find(const ProdTable<void> &t, unsigned char *codes, int n,
+                            const BinLimits &lim, int *row_nz, RowRun *found, RowRun *runs,
+                            const RunTable &rt, int *sym_sub, cudaStream_t s);
+// One program for each of nprog patterns (run_prog_bytes() each).
+size_t run_prog_bytes();
+cudaError_t launch_run_progs(const ProdTable<void> &t, const RowRun *found, const RunTable &rt,
+                             int nprog, bool fp32, void *progs, int *err, cudaStream_t s);
+// Each run's program, its rows' counts in row_nz (if not null), and the
+// members' numeric bins counted in num_sub.
+cudaError_t launch_run_counts(RowRun *runs, const int (&nruns)[2], int cap, const RunTable &rt,
+                              const void *progs, int *row_nz, const int *crpt,
+                              const BinLimits &lim, int *num_sub, cudaStream_t s);
+// Numeric phase of every run. ticket: two zeroed counters.
+cudaError_t launch_numeric_run(const ProdTable<double> &t, const RowRun *runs,
+                               const int (&nruns)[2], int cap, const void *progs, const int *crpt,
+                               int *ccol, double *cval, int *err, int *ticket, cudaStream_t s);
+cudaError_t launch_numeric_comp_run(const ProdTable<float> &t, const RowRun *runs,
+                                    const int (&nruns)[2], int cap, const void *progs,
+                                    const int *crpt, int *ccol, double *cval, int nmax, int *redo,
+                                    int *max_deg, int *err, int *ticket, cudaStream_t s);
 }  // namespace nspb

@@ -83,13 +83,41 @@ cudaError_t launch_check_sorted_table(const Operands<void> *ops, int nprod, int 
 // a power-law row of 10^4 entries does not leave one lane group walking it.
 constexpr int kRowinfoLong = 1024;
 
-template <int GA, bool MULTI>
-__global__ void __launch_bounds__(256)
-    k_rowinfo(const ProdTable<void> src, int n, const BinLimits lim,
+// Counts, bins and, where runs are wanted, the links between rows: a thread a
+// row over columns staged in shared memory (common.cuh). On structured
+// operands the threads of a warp then gather neighbouring entries of B's row
+// pointer; a group of lanes a row waited for pointer, columns and gather in
+// turn (370 us on the 27-point 128^3 stencil, 150 us on the power-law 1M
+// matrix). Rows of more than kInfoSerial entries are left to the whole warp,
+// those of more than kRowinfoLong to k_rowinfo_long.
+constexpr int kInfoSerial = 64;
+
+template <bool MULTI>
+__global__ void __launch_bounds__(kTileThreads)
+    k_rowinfo(const ProdTable<void> src, int n, int tile, const BinLimits lim,
               int *__restrict__ row_nz, int64_t *__restrict__ row_ip,
               int *__restrict__ sym_counts,
               unsigned long long *__restrict__ total_ip, int *__restrict__ flags,
-              int *__restrict__ long_list, int *__restrict__ long_count) {
+              int *__restrict__ long_list, int *__restrict__ long_count, const RunScan runs) {
+  // Rows that repeat an earlier row (runs.codes): row r takes the code
+  // s | sigma << 2 when its A columns are those of row r - s all plus sigma
+  // and every B row it reads is the B row sigma before it moved by one and
+  // the same column shift; s is the smallest such distance, one with sigma = s
+  // before the others (with two unknowns a node, every other row is also its
+  // predecessor moved by two, which no run could follow). Only lags that two
+  // fifths of B's rows have are looked at, so that operands without structure
+  // pay for the counts alone.
+  int lags = 0;
+  if (runs.codes) {
+    for (int g = 1; g <= kMaxLag; ++g)
+      if (5LL * __ldg(runs.lag_count + g) >= 2LL * runs.brows) lags |= 1 << g;
+    if (runs.codes_only && !lags) {
+      for (long long r = blockIdx.x * (long long)kTileThreads + threadIdx.x; r < n;
+           r += gridDim.x * (long long)kTileThreads)
+        runs.codes[r] = 0;
+      return;
+    }
+  }
   // With flags (B is A): the order of every row read here is checked too,
   // which is the B check of launch_check_sorted without a second read.
   // persistent grid: bin counts and the total accumulate in shared memory and
@@ -97,40 +125,177 @@ __global__ void __launch_bounds__(256)
   // block add into the same dozen counters)
   __shared__ int hist[kSymBins];
   __shared__ unsigned long long s_total;
+  __shared__ int cols[kTileWords];
+  __shared__ int rp[kTileThreads + kMaxLag + 1];  // row starts from three rows before the tile
   if (threadIdx.x < kSymBins) hist[threadIdx.x] = 0;
   if (threadIdx.x == 0) s_total = 0ull;
   __syncthreads();
-  auto tile = cg::tiled_partition<GA>(cg::this_thread_block());
-  const int lane = tile.thread_rank();
-  constexpr int kGroups = 256 / GA;
+  const int lane = threadIdx.x & 31;
   unsigned long long my_total = 0;
   int bad = 0;
-  for (int row = blockIdx.x * kGroups + (int)threadIdx.x / GA; row < n;
-       row += gridDim.x * kGroups) {
+  for (long long first = (long long)blockIdx.x * tile; first < n;
+       first += (long long)gridDim.x * tile) {
+    const int r0 = (int)first, nr = min(tile, n - r0);
+    const int q = threadIdx.x, row = r0 + q;
     Operands<void> o;
-    const int lr = prod_row<MULTI>(src, row, o);
-    const int a0 = o.arpt[lr], a1 = o.arpt[lr + 1];
-    if (long_list && a1 - a0 > kRowinfoLong) {  // left to k_rowinfo_long
-      if (lane == 0) long_list[atomicAdd(long_count, 1)] = row;
-      continue;
+    int lr = 0, a0 = 0, a1 = 0, e0 = 0, skew = 31;
+    bool staged = false;
+    // a tile with rows of two products is not staged and finds no links
+    const bool split = MULTI && __ldg(src.prod_of_row + r0) != __ldg(src.prod_of_row + r0 + nr - 1);
+    __syncthreads();  // the last tile is read
+    if (!split) {
+      const int lr0 = prod_row<MULTI>(src, r0, o);
+      for (int i = threadIdx.x; i <= nr + kMaxLag; i += kTileThreads)
+        rp[i] = __ldg(o.arpt + max(lr0 - kMaxLag + i, 0));
+      __syncthreads();
+      lr = lr0 + q;
+      e0 = rp[kMaxLag - min(kMaxLag, lr0)];
+      const int e1 = rp[nr + kMaxLag];
+      staged = e1 - e0 <= kTileCols;
+      if (staged) {
+        skew = tile_skew(rp[nr / 2 + kMaxLag + 1] - rp[nr / 2 + kMaxLag]);
+        tile_stage(o.acol, e0, e1, skew, cols);
+        __syncthreads();
+      }
+      if (q < nr) {
+        a0 = rp[q + kMaxLag];
+        a1 = rp[q + kMaxLag + 1];
+      }
+    } else if (q < nr) {
+      lr = prod_row<MULTI>(src, row, o);
+      a0 = __ldg(o.arpt + lr);
+      a1 = __ldg(o.arpt + lr + 1);
     }
-    long long ip = 0;
-    for (int j = a0 + lane; j < a1; j += GA) {
-      const int k = ld_stream(o.acol + j);
-      ip += o.brpt[k + 1] - o.brpt[k];
-      // each entry against its predecessor, read directly: no dependence
-      // between rounds, so long rows keep their loads in flight
-      if (flags && j > a0 && k <= __ldg(o.acol + j - 1)) bad = 1;
-    }
-    ip = cg::reduce(tile, ip, cg::plus<long long>());
-    if (lane == 0) {
+    const int na = a1 - a0;
+    const bool listed = long_list && na > kRowinfoLong;  // left to k_rowinfo_long
+    with_cols(staged, skew, cols, e0, o.acol, [&](auto col) {
+      // sigma of the link to the row g before, by A's columns; 0: none
+      auto a_link = [&](int g) {
+        const int p0 = rp[q + kMaxLag - g];
+        if (lr < g || rp[q + kMaxLag - g + 1] - p0 != na) return 0;
+        const int sigma = col(a0) - col(p0);
+        if (sigma < 1 || sigma > kMaxLag || !((lags >> sigma) & 1)) return 0;
+        if (runs.same) {
+          const int d = __ldg(&o.bdel[(long long)(g - 1) * o.brows + lr].x);
+          return d == sigma ? sigma : 0;
+        }
+        if (col(a0 + na - 1) - col(p0 + na - 1) != sigma) return 0;
+        int off = 0;
+#pragma unroll 4
+        for (int j = 1; j < na; ++j) off |= (col(a0 + j) - col(p0 + j)) ^ sigma;
+        return off ? 0 : sigma;
+      };
+      int code = 0;
+      if (lags && !split && na > 0 && na <= kRunMaxA) {
+        for (int g = 1; g <= kMaxLag; ++g) {
+          const int sigma = a_link(g);
+          if (sigma && (!code || sigma == g)) {
+            code = g | sigma << 2;
+            if (sigma == g) break;
+          }
+        }
+      }
+      // products, and whether every B row is the one sigma before it moved by
+      // one shift. With runs B's lengths come with its shifts, one gather for both.
+      long long ip = 0;
+      int wrong = 0;  // the row's own order, used when B is A
+      auto b_link = [&](int sigma, bool &linked) {
+        const int2 *del = o.bdel + (long long)(sigma - 1) * o.brows;
+        int lo = 0x7fffffff, hi = (int)0x80000000;
+        long long sum = 0;
+        int prev = -1;
+        bool ok = true;
+#pragma unroll 8
+        for (int j = 0; j < na; ++j) {
+          const int k = col(a0 + j);
+          const int2 x = __ldg(del + k);
+          wrong |= k <= prev;
+          prev = k;
+          sum += x.y;
+          ok = ok && x.x != kNoShift;
+          if (x.x != kAnyShift) {
+            lo = min(lo, x.x);
+            hi = max(hi, x.x);
+          }
+        }
+        linked = ok && lo == hi;
+        return sum;
+      };
+      bool linked = false;
+      if (code) {
+        ip = b_link(code >> 2, linked);
+      } else if (na <= kInfoSerial) {
+        if (runs.codes) {
+#pragma unroll 8
+          for (int j = 0, prev = -1; j < na; ++j) {
+            const int k = col(a0 + j);
+            ip += __ldg(&o.bdel[k].y);
+            wrong |= k <= prev;
+            prev = k;
+          }
+        } else {
+#pragma unroll 4
+          for (int j = 0; j < na; ++j) {
+            const int k = col(a0 + j);
+            ip += __ldg(o.brpt + k + 1) - __ldg(o.brpt + k);
+            if (flags) wrong |= j > 0 && k <= col(a0 + j - 1);
+          }
+        }
+      }
+      if (flags) bad |= wrong;
+      // longer rows, a warp a row
+      unsigned todo = __ballot_sync(0xffffffffu, na > kInfoSerial && !code && !listed);
+      while (todo) {
+        const int w = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        const int b0 = __shfl_sync(0xffffffffu, a0, w), b1 = __shfl_sync(0xffffffffu, a1, w);
+        const int *acol = o.acol, *brpt = o.brpt;
+        if (MULTI && split) {
+          acol = reinterpret_cast<const int *>(
+              __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(acol), w));
+          brpt = reinterpret_cast<const int *>(
+              __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(brpt), w));
+        }
+        auto at = [&](int j) { return MULTI && split ? __ldg(acol + j) : col(j); };
+        long long sum = 0;
+        for (int j = b0 + lane; j < b1; j += 32) {
+          const int k = at(j);
+          sum += __ldg(brpt + k + 1) - __ldg(brpt + k);
+          if (flags) bad |= j > b0 && k <= at(j - 1);
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (lane == w) ip = sum;
+      }
+      if (q >= nr) return;
+      if (listed) {
+        long_list[atomicAdd(long_count, 1)] = row;
+        if (runs.codes) runs.codes[row] = 0;
+        return;
+      }
+      if (code && (ip <= 0 || ip > kRunMaxIp)) code = 0;
+      if (code && !linked) {
+        const int tried = code;
+        code = 0;
+        for (int g = 1; g <= kMaxLag; ++g) {  // another distance, the same order of choice
+          const int sigma = a_link(g);
+          if (!sigma || (g | sigma << 2) == tried || (code && sigma != g)) continue;
+          b_link(sigma, linked);
+          if (!linked) continue;
+          code = g | sigma << 2;
+          if (sigma == g) break;
+        }
+      }
       const int ub = (int)(ip < (long long)o.ncols ? ip : (long long)o.ncols);
       row_nz[row] = ub;
       if (row_ip) row_ip[row] = ip;
       if (ub > 0) atomicAdd(&hist[sym_bin(ub, lim)], 1);
       my_total += (unsigned long long)ip;
-    }
+      if (runs.codes) runs.codes[row] = (unsigned char)code;
+    });
   }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) my_total += __shfl_xor_sync(0xffffffffu, my_total, d);
   if (lane == 0 && my_total) atomicAdd(&s_total, my_total);
   if (__syncthreads_or(bad) && flags && threadIdx.x == 0) atomicOr(flags, B_UNSORTED);
   if (threadIdx.x < kSymBins && hist[threadIdx.x])
@@ -190,25 +355,16 @@ cudaError_t launch_rowinfo(const ProdTable<void> &t, int n, int64_t a_nnz, const
                            int *row_nz,
                            int64_t *row_ip, int *sym_counts,
                            unsigned long long *total_ip, int *flags, int *long_list,
-                           int *long_count, cudaStream_t s) {
+                           int *long_count, const RunScan &runs, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const double avg = (double)a_nnz / (double)n;
-  const int ga = avg > 24.0 ? 32 : avg > 12.0 ? 16 : avg > 6.0 ? 8 : 4;
-  const int grid = (int)std::min<int64_t>(((int64_t)n * ga + 255) / 256,
-                                          (int64_t)dev_info().sms * 8);
+  const int tile = tile_rows(avg);
+  const int grid = (int)std::min<int64_t>(((int64_t)n + tile - 1) / tile,
+                                          (int64_t)dev_info().sms * 6);
   const bool multi = t.prod_of_row != nullptr;
-#define NSPB_RI(GA)                                                                         \
-  (multi ? k_rowinfo<GA, true><<<grid, 256, 0, s>>>(t, n, lim, row_nz, row_ip, sym_counts, total_ip, \
-                                                    flags, long_list, long_count)           \
-         : k_rowinfo<GA, false><<<grid, 256, 0, s>>>(t, n, lim, row_nz, row_ip, sym_counts,       \
-                                                     total_ip, flags, long_list, long_count))
-  switch (ga) {
-    case 32: NSPB_RI(32); break;
-    case 16: NSPB_RI(16); break;
-    case 8: NSPB_RI(8); break;
-    default: NSPB_RI(4); break;
-  }
-#undef NSPB_RI
+  auto kern = multi ? k_rowinfo<true> : k_rowinfo<false>;
+  kern<<<grid, kTileThreads, 0, s>>>(t, n, tile, lim, row_nz, row_ip, sym_counts, total_ip, flags,
+                                     long_list, long_count, runs);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !long_list) return e;
   auto klong = multi ? k_rowinfo_long<true> : k_rowinfo_long<false>;
@@ -226,7 +382,8 @@ cudaError_t launch_rowinfo(const ProdTable<void> &t, int n, int64_t a_nnz, const
 // rely on (rows of a structured grid repeat their neighbours' pattern).
 __global__ void __launch_bounds__(1024)
     k_perm(const int *__restrict__ key, int n, int kind, BinOffsets off, const BinLimits lim,
-           int *__restrict__ cursor, int *__restrict__ perm) {
+           const unsigned char *__restrict__ member, int *__restrict__ cursor,
+           int *__restrict__ perm) {
   __shared__ int wcnt[16][33];  // [bin][warp]: rows, then the warp's offset in the block
   __shared__ int base[16];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -235,7 +392,7 @@ __global__ void __launch_bounds__(1024)
   int b = -1;
   if (i < n) {
     const int k = kind == 0 ? key[i] : key[i + 1] - key[i];
-    if (k > 0) b = kind == 0 ? sym_bin(k, lim) : num_bin(k, lim);
+    if (k > 0 && !(member && member[i])) b = kind == 0 ? sym_bin(k, lim) : num_bin(k, lim);
   }
   __syncthreads();
   const unsigned peers = __match_any_sync(0xffffffffu, b);
@@ -258,9 +415,9 @@ __global__ void __launch_bounds__(1024)
 }
 
 cudaError_t launch_perm(const int *key, int n, int kind, BinOffsets offsets, const BinLimits &lim,
-                        int *cursor, int *perm, cudaStream_t s) {
+                        const unsigned char *member, int *cursor, int *perm, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_perm<<<(n + 1023) / 1024, 1024, 0, s>>>(key, n, kind, offsets, lim, cursor, perm);
+  k_perm<<<(n + 1023) / 1024, 1024, 0, s>>>(key, n, kind, offsets, lim, member, cursor, perm);
   return cudaGetLastError();
 }
 

@@ -156,12 +156,13 @@ int Call::init(const nspb_csr_in *a, const nspb_csr_in *b, const nspb_opts *o) {
   fill(B, b);
   n = A.nrows;
   t64 = ProdTable<double>{};
-  t64.one = Operands<double>{A.rpt, A.col, A.val, B.rpt, B.col, B.val, B.ncols, B.nrows};
+  t64.one = Operands<double>{A.rpt, A.col, A.val, B.rpt, B.col, B.val, B.ncols, B.nrows, nullptr};
   t32 = ProdTable<float>{};
-  t32.one = Operands<float>{A.rpt, A.col, A.val32, B.rpt, B.col, B.val32, B.ncols, B.nrows};
-  info = ProdInfo{n, B.ncols, 1, B.nrows};
+  t32.one = Operands<float>{A.rpt, A.col, A.val32, B.rpt, B.col, B.val32, B.ncols, B.nrows, nullptr};
+  info = ProdInfo{n, B.ncols, 1, B.nrows, B.nrows, false};
   lim = bin_limits(opts.sym_fill_pct, opts.num_fill_pct);
   a_nnz = A.nnz;
+  b_nnz = B.nnz;
   table = false;
   ops = nullptr;
   if (opts.timing) {
@@ -199,8 +200,9 @@ size_t Call::scratch_bytes() {
   const size_t nn = (size_t)std::max(n, 1);
   off_row_nz = 0;
   off_perm = align256(off_row_nz + (nn + 1) * 4);
-  off_counters = align256(off_perm + nn * 4);
-  off_tiles = align256(off_counters + sizeof(DevCounters));
+  off_slots = align256(off_perm + nn * 4);
+  off_counters = align256(off_slots + 2 * kRunSlots * 4);
+  off_tiles = align256(off_counters + sizeof(DevCounters) + kRunSlots * 4);
   const size_t tiles = (size_t)scan_tiles(n);
   ws_bytes = align256(off_tiles + tiles * 8);
   return ws_bytes;
@@ -220,7 +222,11 @@ int Call::alloc_scratch() {
   perm = reinterpret_cast<int *>(ws + off_perm);
   ctr = reinterpret_cast<DevCounters *>(ws + off_counters);
   tile_state = reinterpret_cast<unsigned long long *>(ws + off_tiles);
-  // counters and scan tile states are contiguous: one memset clears both
+  rtab.head = &ctr->run;
+  rtab.rep = reinterpret_cast<int *>(ctr + 1);
+  rtab.prog_of = reinterpret_cast<int *>(ws + off_slots);
+  rtab.run_of = rtab.prog_of + kRunSlots;
+  // counters, pattern table and scan tile states are contiguous: one memset clears them
   cudaError_t e = cudaMemsetAsync(ws + off_counters, 0, ws_bytes - off_counters, s);
   if (e != cudaSuccess) return cuda_fail(e);
   return NSPB_OK;
@@ -229,6 +235,7 @@ int Call::alloc_scratch() {
 Call::~Call() {
   if (ws && !ws_external) scratch_free(ws, s);
   if (map_block) scratch_free(map_block, s);
+  drop_runs();
   for (auto &e : ev)
     if (e) cudaEventDestroy(e);
 }
@@ -280,6 +287,70 @@ static BinOffsets offsets_of(const int *counts, int nb, int *nonempty, int *tota
   return o;
 }
 
+// Row runs are looked for when the caller leaves the choice of the row kernels
+// to the library and A's rows are short enough on average for runs to hold
+// most of them. The search costs a pass over B's columns and six launches, so a
+// product of fewer than about 24 million intermediate products (A's entries
+// times B's mean row) does without, unless row_kernel is 8. Measured, runs
+// against none: 27-point 40^3 (42 M) 379 vs 519 us, 32^3 (21 M) 288 vs 317, 24^3
+// (8.5 M) 268 vs 222, R (A P) of 60^3 (11 M) 401 vs 360.
+bool Call::runs_wanted() const {
+  if (!allow_runs || family() != 0 || (opts.row_kernel & kNoRowTemplates)) return false;
+  if (n < 2 * kRunMin || a_nnz > (int64_t)kRunMaxA * n || (table && !info.bdel)) return false;
+  if ((opts.row_kernel & 0xff) == 8) return true;
+  return info.brows > 0 && (double)a_nnz * (double)b_nnz >= 24e6 * (double)info.brows;
+}
+
+int Call::alloc_runs() {
+  const size_t cap = (size_t)run_capacity(n) * sizeof(RowRun);
+  const size_t o_found = align256((size_t)n), o_runs = align256(o_found + cap);
+  const size_t o_del = align256(o_runs + cap);
+  const size_t bytes = o_del + (table ? 0 : (size_t)kMaxLag * std::max(B.nrows, 1) * sizeof(int2));
+  int st = scratch_alloc(reinterpret_cast<void **>(&run_block), bytes, s);
+  if (st) return st;
+  member = reinterpret_cast<unsigned char *>(run_block);
+  found = reinterpret_cast<RowRun *>(run_block + o_found);
+  runs = reinterpret_cast<RowRun *>(run_block + o_runs);
+  if (!table) t64.one.bdel = t32.one.bdel = reinterpret_cast<int2 *>(run_block + o_del);
+  return NSPB_OK;
+}
+
+int Call::build_programs() {
+  for (int c = 0; c < 2; ++c) nruns[c] = run_block ? h.run.nruns[c] : 0;
+  use_runs = nruns[0] + nruns[1] > 0;
+  if (!use_runs) return NSPB_OK;
+  int st = scratch_alloc(&progs, (size_t)h.run.nprog * run_prog_bytes(), s);
+  if (st) return st;
+  const cudaError_t e = launch_run_progs(structure_of(t64), found, rtab, h.run.nprog,
+                                         fp32_inputs(opts.precision), progs, &ctr->err, s);
+  if (e != cudaSuccess) return cuda_fail(e);
+  ++launches;
+  return NSPB_OK;
+}
+
+void Call::drop_runs() {
+  if (run_block) scratch_free(run_block, s);
+  if (progs) scratch_free(progs, s);
+  run_block = nullptr;
+  progs = nullptr;
+  t64.one.bdel = t32.one.bdel = nullptr;
+  use_runs = false;
+  nruns[0] = nruns[1] = 0;
+}
+
+// same: B is A, whose order the row walk of k_rowinfo checks.
+cudaError_t Call::check_b(bool same) {
+  if (run_block) {
+    ++launches;
+    return launch_brow_delta(structure_of(t64), info, b_nnz, ctr->lag_count,
+                             opts.assume_sorted || same ? nullptr : &ctr->flags, s);
+  }
+  if (opts.assume_sorted || same) return cudaSuccess;
+  ++launches;
+  return table ? launch_check_sorted_table(ops, info.nprod, info.max_brows, &ctr->flags, s)
+               : launch_check_sorted(B, &ctr->flags, s);
+}
+
 // Steps 1-5: C.rowptr and nnz(C). crpt must hold n+1 ints.
 int Call::symbolic(int *crpt, int64_t *nnz_out) {
   cudaError_t e;
@@ -295,29 +366,43 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
   // B = A (the same arrays): the row walk of k_rowinfo checks B's order too
   const bool same = !table && A.rpt == B.rpt && A.col == B.col && A.nrows == B.nrows &&
                     A.nnz == B.nnz;
-  if (!opts.assume_sorted && !same) {
-    e = table ? launch_check_sorted_table(ops, info.nprod, info.max_brows, &ctr->flags, s)
-              : launch_check_sorted(B, &ctr->flags, s);
-    if (e != cudaSuccess) return cuda_fail(e);
-    ++launches;
-  }
+  if (runs_wanted() && alloc_runs()) drop_runs();  // no memory for them: every row on its own
+  if ((e = check_b(same)) != cudaSuccess) return cuda_fail(e);
+  RunScan scan;
+  if (run_block) scan = RunScan{member, ctr->lag_count, info.brows, false, same};
   // perm is free until the bins are permuted: it holds the long-row list here
   if ((e = launch_rowinfo(structure_of(t64), n, a_nnz, lim, row_nz, nullptr, ctr->sym_counts,
                           &ctr->total_ip,
                           !opts.assume_sorted && same ? &ctr->flags : nullptr, perm,
-                          &ctr->long_rows, s)) != cudaSuccess)
+                          &ctr->long_rows, scan, s)) != cudaSuccess)
     return cuda_fail(e);
+  if (run_block) {
+    if ((e = launch_run_find(structure_of(t64), member, n, lim, row_nz, found, runs, rtab,
+                             ctr->sym_sub, s)) != cudaSuccess)
+      return cuda_fail(e);
+    launches += 2;
+  }
   ++launches;
   mark(1);
   if ((st = fetch_counters())) return st;
   b_sorted = opts.assume_sorted || !(h.flags & B_UNSORTED);
   intprod = (int64_t)h.total_ip;
+  if ((st = build_programs()) == NSPB_ERR_ALLOC) {  // no memory for them: without runs
+    drop_runs();
+    allow_runs = false;
+    if (!ws_external) scratch_free(ws, s);
+    ws = nullptr;
+    return symbolic(crpt, nnz_out);
+  }
+  if (st) return st;
+  int todo[16];  // rows of each bin to be counted: those that no run serves
+  for (int b = 0; b < 16; ++b) todo[b] = h.sym_counts[b] - (use_runs ? h.sym_sub[b] : 0);
   // the mean length of the B rows actually read, weighted by how often A reads
   // them: a block-diagonal batch mixes products whose B rows differ
   if (!(opts.group_lanes == 8 || opts.group_lanes == 16 || opts.group_lanes == 32) && a_nnz > 0)
     lanes = pick_lanes((double)intprod / (double)a_nnz, (double)a_nnz / (double)n, n);
   int nonempty = 0, binned = 0;
-  BinOffsets off = offsets_of(h.sym_counts, kSymBins, &nonempty, &binned);
+  BinOffsets off = offsets_of(todo, kSymBins, &nonempty, &binned);
   const bool direct = nonempty == 1 && binned == n;
   // entry maps: a stride of the bin's row limit (products) per row
   long long map_bin_off[kSymGroupBins] = {};
@@ -329,7 +414,7 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
       // quads of the map take at most 4/3 of a byte per product, plus alignment
       map_stride[b] = (int)(((long long)lim.sym[b] * 3 / 2 + 16 + 15) & ~15LL);
       map_bin_off[b] = total;
-      total += (long long)h.sym_counts[b] * map_stride[b];
+      total += (long long)todo[b] * map_stride[b];
     }
     const size_t head = align256((size_t)n * 4);
     // row templates of one product check B rows by their shift bits
@@ -345,22 +430,23 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
       map = static_cast<unsigned char *>(map_block) + head + bits;
       use_map = true;
       if (bshift) {
-        if ((e = launch_brow_shift(B.rpt, B.col, B.nrows, bshift, s)) != cudaSuccess)
-          return cuda_fail(e);
+        e = run_block ? launch_shift_bits(t64.one.bdel, B.nrows, bshift, s)
+                      : launch_brow_shift(B.rpt, B.col, B.nrows, bshift, s);
+        if (e != cudaSuccess) return cuda_fail(e);
         ++launches;
       }
     }
   }
   mark(2);
   if (!direct && binned > 0) {
-    if ((e = launch_perm(row_nz, n, 0, off, lim, ctr->cursor_sym, perm, s)) != cudaSuccess)
+    if ((e = launch_perm(row_nz, n, 0, off, lim, nullptr, ctr->cursor_sym, perm, s)) != cudaSuccess)
       return cuda_fail(e);
     ++launches;
-    if ((e = order_block_bins(row_nz, 0, h.sym_counts, kSymGroupBins, kSymBins, off)) != cudaSuccess)
+    if ((e = order_block_bins(row_nz, 0, todo, kSymGroupBins, kSymBins, off)) != cudaSuccess)
       return cuda_fail(e);
   }
   for (int b = 0; b < kSymBins; ++b) {
-    const int c = h.sym_counts[b];
+    const int c = todo[b];
     if (c <= 0) continue;
     const int *rows = direct ? nullptr : perm + off.v[b];
     if (use_map) {
@@ -380,6 +466,12 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
     if (e != cudaSuccess) return cuda_fail(e);
     ++launches;
   }
+  if (use_runs) {
+    if ((e = launch_run_counts(runs, nruns, (int)run_capacity(n), rtab, progs, row_nz, nullptr, lim,
+                               ctr->num_sub, s)) != cudaSuccess)
+      return cuda_fail(e);
+    ++launches;
+  }
   mark(3);
   if ((e = launch_scan(row_nz, n, crpt, &ctr->total_nnz, tile_state, &ctr->tile_ctr, lim,
                        ctr->num_counts, &ctr->err, s)) != cudaSuccess)
@@ -388,6 +480,7 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
   mark(4);
   if ((st = fetch_counters())) return st;
   num_counts_ready = true;
+  for (int b = 0; b < 16; ++b) run_rows[b] = use_runs ? h.num_sub[b] : 0;
   if (use_map && (h.flags & MAP_OVERFLOW)) {  // a row outgrew its stride: no map
     use_map = false;
     scratch_free(map_block, s);
@@ -406,15 +499,18 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
   cudaError_t e;
   if (n == 0) return NSPB_OK;
   int nonempty = 0, binned = 0;
-  BinOffsets off = offsets_of(h.num_counts, kNumBins, &nonempty, &binned);
-  if (binned == 0) return NSPB_OK;
+  int todo[16];  // rows of each bin that no run serves
+  for (int b = 0; b < 16; ++b) todo[b] = h.num_counts[b] - run_rows[b];
+  BinOffsets off = offsets_of(todo, kNumBins, &nonempty, &binned);
+  if (binned == 0 && !use_runs) return NSPB_OK;
   const bool direct = nonempty == 1 && binned == n;
   mark(5);
-  if (!direct) {
-    if ((e = launch_perm(crpt, n, 1, off, lim, ctr->cursor_num, perm, s)) != cudaSuccess)
+  if (!direct && binned > 0) {
+    if ((e = launch_perm(crpt, n, 1, off, lim, use_runs ? member : nullptr, ctr->cursor_num, perm,
+                         s)) != cudaSuccess)
       return cuda_fail(e);
     ++launches;
-    if ((e = order_block_bins(crpt, 1, h.num_counts, kNumGroupBins, kNumBins, off)) != cudaSuccess)
+    if ((e = order_block_bins(crpt, 1, todo, kNumGroupBins, kNumBins, off)) != cudaSuccess)
       return cuda_fail(e);
   }
   // fp32 inputs: rows of at most nmax A entries accumulate in fp32 pairs, the
@@ -422,8 +518,18 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
   const bool comp = fp32_inputs(opts.precision);
   const int nmax = opts.precision == NSPB_PREC_FP32_COMP ? comp_nmax(opts.comp_tol) : 0;
   const bool staged = use_staged();
+  if (use_runs) {
+    const int cap = (int)run_capacity(n);
+    e = comp ? launch_numeric_comp_run(t32, runs, nruns, cap, progs, crpt, ccol, cval, nmax,
+                                       &ctr->redo_count, &ctr->max_comp_deg, &ctr->err,
+                                       &ctr->ticket[30], s)
+             : launch_numeric_run(t64, runs, nruns, cap, progs, crpt, ccol, cval, &ctr->err,
+                                  &ctr->ticket[30], s);
+    if (e != cudaSuccess) return cuda_fail(e);
+    launches += (nruns[0] > 0) + (nruns[1] > 0);
+  }
   for (int b = 0; b < kNumBins; ++b) {
-    const int c = h.num_counts[b];
+    const int c = todo[b];
     if (c <= 0) continue;
     const int *rows = direct ? nullptr : perm + off.v[b];
     int *ticket = &ctr->ticket[16 + b];
@@ -481,7 +587,7 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
 // 96^3 stencil (4.5 on 16 lanes), and on random products of 4..32 entries
 // a row, 3.2 vs 3.0 ms (18 on 32 lanes, against the hash-sort kernels).
 bool Call::map_wanted() const {
-  const int k = opts.row_kernel & 0xff;
+  const int k = family();
   if (!allow_map || !(k == 0 || k == 7)) return false;
   if (!b_sorted || n <= 0 || a_nnz <= 0) return false;
   if (info.max_ncols > kMapMaxCols) return false;
@@ -497,16 +603,38 @@ int Call::prepare_numeric(const int *crpt) {
   int st = alloc_scratch();
   if (st) return st;
   cudaError_t e;
-  if (!opts.assume_sorted) {
-    e = table ? launch_check_sorted_table(ops, info.nprod, info.max_brows, &ctr->flags, s)
-              : launch_check_sorted(B, &ctr->flags, s);
-    if (e != cudaSuccess) return cuda_fail(e);
+  if (runs_wanted() && alloc_runs()) drop_runs();
+  if ((e = check_b(false)) != cudaSuccess) return cuda_fail(e);
+  if (run_block) {
+    // the runs again (the symbolic phase was another call's); operands without
+    // structure skip the row walk
+    const bool same = !table && A.rpt == B.rpt && A.col == B.col && A.nrows == B.nrows &&
+                      A.nnz == B.nnz;
+    const RunScan scan{member, ctr->lag_count, info.brows, true, same};
+    if ((e = launch_rowinfo(structure_of(t64), n, a_nnz, lim, row_nz, nullptr, ctr->sym_counts,
+                            &ctr->total_ip, nullptr, perm, &ctr->long_rows, scan, s)) !=
+            cudaSuccess ||
+        (e = launch_run_find(structure_of(t64), member, n, lim, row_nz, found, runs, rtab,
+                             ctr->sym_sub, s)) != cudaSuccess)
+      return cuda_fail(e);
+    launches += 3;
   }
   if ((e = launch_num_hist(crpt, n, lim, ctr->num_counts, s)) != cudaSuccess) return cuda_fail(e);
-  launches += opts.assume_sorted ? 1 : 2;
+  ++launches;
   if ((st = fetch_counters())) return st;
   b_sorted = opts.assume_sorted || !(h.flags & B_UNSORTED);
   num_counts_ready = true;
+  intprod = (int64_t)h.total_ip;  // 0 where the row walk was skipped
+  if ((st = build_programs()) == NSPB_ERR_ALLOC) drop_runs();
+  else if (st) return st;
+  if (use_runs) {
+    if ((e = launch_run_counts(runs, nruns, (int)run_capacity(n), rtab, progs, nullptr, crpt, lim,
+                               ctr->num_sub, s)) != cudaSuccess)
+      return cuda_fail(e);
+    ++launches;
+    if ((st = fetch_counters())) return st;
+    for (int b = 0; b < 16; ++b) run_rows[b] = h.num_sub[b];
+  }
   return NSPB_OK;
 }
 
@@ -761,7 +889,7 @@ int nspb_intprod(const nspb_csr_in *A, const nspb_csr_in *B, int64_t *d_row_ip, 
   cudaError_t e = launch_rowinfo(structure_of(call.t64), call.n, call.a_nnz, call.lim, call.row_nz,
                                  d_row_ip, call.ctr->sym_counts,
                                  &call.ctr->total_ip, nullptr, call.perm, &call.ctr->long_rows,
-                                 call.s);
+                                 RunScan(), call.s);
   if (e != cudaSuccess) return call.cuda_fail(e);
   if ((st = call.fetch_counters())) return st;
   if (total) *total = (int64_t)call.h.total_ip;

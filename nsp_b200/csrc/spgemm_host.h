@@ -27,7 +27,11 @@ struct DevCounters {
   int long_rows;     // rows listed for the block-per-row intermediate-product count
   int pad;
   int ticket[32];    // row tickets of the block-per-row launches (symbolic
-                     // bin b at b, numeric bin b at 16 + b)
+                     // bin b at b, numeric bin b at 16 + b; the runs at 30, 31)
+  int lag_count[4];  // B rows with a column shift at lag 1, 2, 3
+  int sym_sub[16];   // rows of each symbolic bin that belong to a run
+  int num_sub[16];   // rows of each numeric bin that do
+  RunHead run;
 };
 
 struct HostStage {
@@ -56,7 +60,7 @@ struct Call {
   // scratch (one stream-ordered block)
   char *ws = nullptr;
   size_t ws_bytes = 0;
-  size_t off_row_nz = 0, off_perm = 0, off_counters = 0, off_tiles = 0;
+  size_t off_row_nz = 0, off_perm = 0, off_slots = 0, off_counters = 0, off_tiles = 0;
   int *row_nz = nullptr;
   int *perm = nullptr;
   DevCounters *ctr = nullptr;
@@ -85,6 +89,26 @@ struct Call {
   unsigned *map_off = nullptr;
   unsigned *bshift = nullptr;  // B row shift bits for the row templates (one product)
   bool map_wanted() const;
+  // Row runs (rowrun.cu): rows that repeat a pattern at a fixed distance are
+  // counted once a run and computed by k_num_run. allow_runs false: entry
+  // points that may not allocate.
+  bool allow_runs = true;
+  bool use_runs = false;
+  int nruns[2] = {0, 0};       // of few, of many products a row
+  char *run_block = nullptr;   // pool block: member flags, runs, B row shifts
+  unsigned char *member = nullptr;
+  RowRun *found = nullptr, *runs = nullptr;
+  RunTable rtab;
+  void *progs = nullptr;       // pool block: one program a pattern
+  int run_rows[16] = {};       // rows of each numeric bin that belong to runs
+  int64_t b_nnz = 0;           // entries of B over all products
+  bool runs_wanted() const;
+  int alloc_runs();
+  void drop_runs();
+  // After the counters are read: the programs of the patterns found.
+  int build_programs();
+  // B's row order and, with runs, its column shifts
+  cudaError_t check_b(bool same);
   // opts.timing: events around rowinfo, symbolic, scan, numeric
   cudaEvent_t ev[8] = {};
   bool timing = false;
@@ -94,8 +118,14 @@ struct Call {
   // staged walk wins on stencils, 1.04x, and 7-point Laplacians, 1.27x, and
   // loses on random and power-law rows, where almost every product is a new
   // entry). Needs B rows strictly increasing.
-  bool use_staged() const {
+  // kernel family asked for: 0 (automatic) for 8, which only turns off the
+  // size rule of the row runs
+  int family() const {
     const int k = opts.row_kernel & 0xff;
+    return k == 8 ? 0 : k;
+  }
+  bool use_staged() const {
+    const int k = family();
     if (k == 2 || k == 3) return true;
     if (k != 0) return false;
     return h.total_nnz > 0 && (double)intprod >= 1.5 * (double)h.total_nnz;

@@ -202,6 +202,20 @@ cudaError_t launch_brow_shift(const int *brpt, const int *bcol, int nb, unsigned
   return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256)
+    k_shift_bits(const int2 *__restrict__ bdel, int nb, unsigned *__restrict__ bits) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool same = k < nb && bdel[k].x != kNoShift;
+  const unsigned w = __ballot_sync(0xffffffffu, same);
+  if ((threadIdx.x & 31) == 0 && k < nb) bits[k >> 5] = w;
+}
+
+cudaError_t launch_shift_bits(const int2 *bdel, int nb, unsigned *bits, cudaStream_t s) {
+  if (nb <= 0) return cudaSuccess;
+  k_shift_bits<<<(nb + 255) / 256, 256, 0, s>>>(bdel, nb, bits);
+  return cudaGetLastError();
+}
+
 // The scalars of a group's template (shared memory keeps them out of the
 // registers the hash walk needs).
 struct TplHead {
