@@ -178,7 +178,12 @@ const char *nspb_version(void);
 const char *nspb_strerror(int status);
 int nspb_last_cuda_error(void);          /* cudaError_t of the last failure  */
 void nspb_default_opts(nspb_opts *opts);
-int nspb_free(void *device_ptr);         /* cudaFree                         */
+/* Releases an output that the library allocated (any cudaMalloc block): waits
+ * for the device and keeps the block for a later output of about its size (at
+ * most a sixteenth of the device's memory in all, while a quarter is free), or
+ * calls cudaFree. cudaFree on such an output works as well.                 */
+int nspb_free(void *device_ptr);
+int nspb_trim(void);                     /* cudaFree of every block kept     */
 int nspb_device_sm_count(int *sms);
 
 /* ---- the product ---------------------------------------------------------- */

@@ -99,6 +99,7 @@ _SIGS = {
     "nspb_last_cuda_error": (C.c_int, []),
     "nspb_default_opts": (None, [P(Opts)]),
     "nspb_free": (C.c_int, [C.c_void_p]),
+    "nspb_trim": (C.c_int, []),
     "nspb_device_sm_count": (C.c_int, [P(C.c_int)]),
     "nspb_spgemm": (C.c_int, [P(CsrIn), P(CsrIn), P(CsrOut), P(Opts), P(Stats)]),
     "nspb_spgemm_symbolic": (C.c_int, [P(CsrIn), P(CsrIn), P(CsrOut), P(Opts), P(Stats)]),

@@ -690,16 +690,6 @@ int Call::finish(nspb_stats *stats) {
   return NSPB_OK;
 }
 
-int alloc_out(void **p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes < 4 ? 4 : bytes);
-  if (e != cudaSuccess) {
-    g_last_cuda = (int)e;
-    cudaGetLastError();
-    return NSPB_ERR_ALLOC;
-  }
-  return NSPB_OK;
-}
-
 }  // namespace nspb
 
 using namespace nspb;
@@ -731,17 +721,6 @@ void nspb_default_opts(nspb_opts *o) {
   std::memset(o, 0, sizeof(*o));
   o->precision = NSPB_PREC_FP64;
   o->comp_tol = 1e-10;
-}
-
-int nspb_free(void *p) {
-  if (!p) return NSPB_OK;
-  cudaError_t e = cudaFree(p);
-  if (e != cudaSuccess) {
-    g_last_cuda = (int)e;
-    cudaGetLastError();
-    return NSPB_ERR_CUDA;
-  }
-  return NSPB_OK;
 }
 
 int nspb_device_sm_count(int *sms) {
