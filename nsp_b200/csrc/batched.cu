@@ -420,7 +420,7 @@ int dev_alloc(T **p, size_t count) {
 int group_numeric(PlanGroup &G, cudaStream_t s) {
   G.call.s = s;
   if (G.call.n == 0) return NSPB_OK;  // no rows: no scratch, nothing to compute
-  cudaError_t e = cudaMemsetAsync(G.call.ctr, 0, sizeof(DevCounters), s);
+  cudaError_t e = cudaMemsetAsync(G.call.ctr, 0, G.call.counter_bytes(), s);
   if (e != cudaSuccess) return plan_fail(e);
   const int *crp = G.multi ? reinterpret_cast<int *>(G.ws_tab + G.h.o_crp) : G.crp;
   return G.call.numeric(crp, G.ccol, G.cval);

@@ -143,22 +143,34 @@ constexpr int kRunMin = 6;         // rows of the shortest run
 struct RowRun {
   int row0;
   int meta;
-  int prog;  // its pattern's slot, then its program
-  int pad;
+  int prog;   // its pattern's slot (-1: dropped), in the final list its program
+  int place;  // among the runs of its pattern
 };
 inline long long run_capacity(long long n) { return n / kRunMin + 1; }
 // The patterns of the runs: a table of representatives (run index + 1, 0:
 // free), the program of each slot and the representative run of each program.
-constexpr int kRunSlots = 1024;
+constexpr int kRunSlots = 4096;
 struct RunHead {
   int nfound;    // runs found
   int nprog;     // patterns among them
   int nruns[2];  // runs kept: of few, of many products a row
+  int nbunch;    // bunches: patterns shared by rows that are in no run
+  int pad[3];
 };
 struct RunTable {
   RunHead *head = nullptr;
   int *rep = nullptr, *prog_of = nullptr, *run_of = nullptr;  // kRunSlots each; rep zeroed
+  // runs of each slot (zeroed); by program: slot | large << 16, first run in the list
+  int *count = nullptr, *slot_of = nullptr, *first = nullptr;
+  // bunches: representative row + 1 and rows of each slot (zeroed), where a
+  // slot's rows are listed (-1: not a bunch), then by bunch: its first row,
+  // rows and place in the list
+  int *brep = nullptr, *bcount = nullptr, *bslot = nullptr;
+  int *brow = nullptr, *brows = nullptr, *bplace = nullptr;
+  // tiles of few and of many products a row before each bunch (kRunSlots + 64 each)
+  int *btiles[2] = {nullptr, nullptr};
 };
+constexpr int kRunTableZeroed = 4, kRunTableRest = 10;  // tables of kRunSlots ints (+ 64)
 
 // fp32 input modes (compensated pairs, or fp64 accumulation of exact products).
 inline bool fp32_inputs(int precision) {
@@ -314,21 +326,43 @@ cudaError_t launch_numeric_comp_map(int bin, int lanes, const ProdTable<float> &
 // shifts found per lag into lag_count[1..3], and (flags not null) B_UNSORTED.
 cudaError_t launch_brow_delta(const ProdTable<void> &t, const ProdInfo &info, int64_t b_nnz,
                               int *lag_count, int *flags, cudaStream_t s);
-// The runs of launch_rowinfo's codes (found: run_capacity(n) entries), their
-// patterns and the list of those kept (runs: small ones from the front, large
-// ones from the back); codes[] becomes the members' flags, row_nz of every
+// The runs of launch_rowinfo's codes (found: run_capacity(n) entries) and
+// their patterns; codes[] becomes the members' flags, row_nz of every
 // member is zeroed and its symbolic bin counted in sym_sub.
 cudaError_t launch_run_find(const ProdTable<void> &t, unsigned char *codes, int n,
-                            const BinLimits &lim, int *row_nz, RowRun *found, RowRun *runs,
+                            const BinLimits &lim, int *row_nz, RowRun *found,
                             const RunTable &rt, int *sym_sub, cudaStream_t s);
-// One program for each of nprog patterns (run_prog_bytes() each).
+// The rows left over by the runs, by pattern: rows with one pattern of
+// products form a bunch (a single row too); slot and list (n ints each) are
+// theirs, the rest as in launch_run_find.
+cudaError_t launch_bunch_find(const ProdTable<void> &t, unsigned char *member, int n,
+                              const BinLimits &lim, int *row_nz, const RunTable &rt, int *slot,
+                              int *list, int *sym_sub, cudaStream_t s);
+// One program for each of nprog patterns of runs and nbunch of bunches, in
+// this order (run_prog_bytes() each).
 size_t run_prog_bytes();
 cudaError_t launch_run_progs(const ProdTable<void> &t, const RowRun *found, const RunTable &rt,
-                             int nprog, bool fp32, void *progs, int *err, cudaStream_t s);
-// Each run's program, its rows' counts in row_nz (if not null), and the
-// members' numeric bins counted in num_sub.
-cudaError_t launch_run_counts(RowRun *runs, const int (&nruns)[2], int cap, const RunTable &rt,
-                              const void *progs, int *row_nz, const int *crpt,
+                             int nprog, int nbunch, bool fp32, void *progs, int *err,
+                             cudaStream_t s);
+// The rows of the bunches get their count (row_nz not null) and are counted as
+// numeric-bin rows that no bin needs.
+cudaError_t launch_bunch_counts(const RunTable &rt, int nprog, int nbunch, const int *list,
+                                const void *progs, int *row_nz, const int *crpt,
+                                const BinLimits &lim, int *num_sub, cudaStream_t s);
+// Numeric phase of the bunches. ticket: two zeroed counters.
+cudaError_t launch_numeric_bunch(const ProdTable<double> &t, const RunTable &rt, int nprog,
+                                 int nbunch, const int *list, const void *progs, const int *crpt,
+                                 int *ccol, double *cval, int *err, int *ticket, cudaStream_t s);
+cudaError_t launch_numeric_comp_bunch(const ProdTable<float> &t, const RunTable &rt, int nprog,
+                                      int nbunch, const int *list, const void *progs,
+                                      const int *crpt, int *ccol, double *cval, int nmax,
+                                      int *redo, int *max_deg, int *err, int *ticket,
+                                      cudaStream_t s);
+// The runs by program (runs: small ones from the front, large ones from the
+// back), their rows' counts in row_nz (if not null), and the members' numeric
+// bins counted in num_sub.
+cudaError_t launch_run_counts(const RowRun *found, int nfound, RowRun *runs, int cap,
+                              const RunTable &rt, const void *progs, int *row_nz, const int *crpt,
                               const BinLimits &lim, int *num_sub, cudaStream_t s);
 // Numeric phase of every run. ticket: two zeroed counters.
 cudaError_t launch_numeric_run(const ProdTable<double> &t, const RowRun *runs,

@@ -24,6 +24,8 @@
 #include "internal.h"
 #include "launch_util.h"
 
+#include <cuda_pipeline.h>
+
 #include <algorithm>
 
 namespace nspb {
@@ -199,7 +201,7 @@ __global__ void __launch_bounds__(kRunBlock)
       }
     }
     if (len >= kRunMin)
-      run[atomicAdd(&s_n, 1)] = RowRun{b0 + first, s | (c >> 2 & 3) << 2 | len << 4, 0, 0};
+      run[atomicAdd(&s_n, 1)] = RowRun{b0 + first, s | (c >> 2 & 3) << 2 | len << 4, -1, 0};
   }
   __syncthreads();
   if (t == 0 && s_n) s_base = atomicAdd(nfound, s_n);
@@ -211,15 +213,16 @@ __global__ void __launch_bounds__(kRunBlock)
 // ---- the programs -----------------------------------------------------------------
 // Two sizes of the numeric kernel: rows of few products leave little to share
 // out among 16 warps, and many small blocks hide the waits between their steps.
+// WARPS compute, LOOK warps look up tiles.
 template <int CLASS>
 struct RunCfg;
 template <>
 struct RunCfg<0> {  // rows of at most kRunSmallIp products
-  static constexpr int WARPS = 8, SMEM = 50 * 1024, MINB = 4;
+  static constexpr int WARPS = 8, LOOK = 2, SMEM = 50 * 1024, MINB = 4;
 };
 template <>
 struct RunCfg<1> {
-  static constexpr int WARPS = 16, SMEM = 108 * 1024, MINB = 2;
+  static constexpr int WARPS = 16, LOOK = 1, SMEM = 110000, MINB = 2;
 };
 constexpr int kRunSmallIp = 256;
 constexpr int kRunRows = 128;  // most rows of a tile
@@ -245,6 +248,9 @@ struct RunProg {
   int dst[kRunMaxA];     // its place
   int rel[kRunMaxIp];    // columns of the row less the first product's
   uint2 word[kRunMaxIp + 32];
+  // bunches: the A entry of every product, products before every A entry
+  unsigned char term[kRunMaxIp];
+  short before[kRunMaxA + 1];
 };
 static_assert(kRunMaxA <= 128 && kRunMaxIp < 2048, "fields of a program word");
 
@@ -281,22 +287,21 @@ __device__ __forceinline__ unsigned run_mix(unsigned a, unsigned b) {
 // Patterns of the runs: a warp a run hashes everything that its program
 // depends on and looks for a run with the same pattern in a table of
 // representatives; a run that finds one is compared with it, value by value.
-// Runs that find no place in the table are dropped and their rows computed
-// like any others. Runs kept are listed by class (small from the front, large
-// from the back of `runs`), their rows marked and taken out of the symbolic bins.
+// Runs that find no place in the table are dropped (prog -1) and their rows
+// computed like any others. Runs kept take a place in their pattern, and their
+// rows are marked and taken out of the symbolic bins.
 template <bool MULTI>
 __global__ void __launch_bounds__(256)
-    k_run_key(const ProdTable<void> src, const RowRun *__restrict__ found,
-              int cap, const BinLimits lim,
-              unsigned char *__restrict__ member, int *__restrict__ row_nz,
-              RowRun *__restrict__ runs, const RunTable rt, int *__restrict__ sym_sub) {
+    k_run_key(const ProdTable<void> src, RowRun *__restrict__ found, const BinLimits lim,
+              unsigned char *__restrict__ member, int *__restrict__ row_nz, const RunTable rt,
+              int *__restrict__ sym_sub) {
   __shared__ int hist[kSymBins];
   if (threadIdx.x < kSymBins) hist[threadIdx.x] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int total = rt.head->nfound;
   for (int q = (blockIdx.x * 256 + threadIdx.x) >> 5; q < total; q += gridDim.x * 8) {
-    RowRun rd = found[q];
+    const RowRun rd = found[q];
     const int s = rd.meta & 3, sigma = rd.meta >> 2 & 3, len = rd.meta >> 4;
     Operands<void> o;
     const int lr = prod_row<MULTI>(src, rd.row0, o);
@@ -347,11 +352,12 @@ __global__ void __launch_bounds__(256)
           const int p = atomicAdd(&rt.head->nprog, 1);
           rt.prog_of[at] = p;
           rt.run_of[p] = q;
+          rt.slot_of[p] = at | (P > kRunSmallIp) << 16;
         }
         break;
       }
       // the same pattern as the representative's?
-      const RowRun other = found[rep - 1];
+      const RowRun other{found[rep - 1].row0, found[rep - 1].meta, 0, 0};
       if ((other.meta >> 2 & 3) != sigma) continue;
       Operands<void> o2;
       const int lr2 = prod_row<MULTI>(src, other.row0, o2);
@@ -388,16 +394,17 @@ __global__ void __launch_bounds__(256)
       }
       if (!diff) slot = at;
     }
-    if (slot < 0) continue;
-    const int large = P > kRunSmallIp;
-    int at = 0;
     if (lane == 0) {
-      at = atomicAdd(&rt.head->nruns[large], 1);
-      rd.prog = slot;
-      runs[large ? cap - 1 - at : at] = rd;
-      const int ub = row_nz[rd.row0];
-      if (ub > 0) atomicAdd(&hist[sym_bin(ub, lim)], len);
+      const int large = P > kRunSmallIp;
+      found[q].prog = slot;
+      if (slot >= 0) {
+        atomicAdd(&rt.head->nruns[large], 1);
+        found[q].place = atomicAdd(rt.count + slot, 1);
+        const int ub = row_nz[rd.row0];
+        if (ub > 0) atomicAdd(&hist[sym_bin(ub, lim)], len);
+      }
     }
+    if (slot < 0) continue;
     __syncwarp();
     for (int m = lane; m < len; m += 32) {
       member[rd.row0 + s * m] = 1;
@@ -410,7 +417,7 @@ __global__ void __launch_bounds__(256)
 }
 
 cudaError_t launch_run_find(const ProdTable<void> &t, unsigned char *codes, int n,
-                            const BinLimits &lim, int *row_nz, RowRun *found, RowRun *runs,
+                            const BinLimits &lim, int *row_nz, RowRun *found,
                             const RunTable &rt, int *sym_sub, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   k_run_list<<<(n + kRunBlock - 1) / kRunBlock, kRunBlock, 0, s>>>(codes, n, found,
@@ -420,7 +427,209 @@ cudaError_t launch_run_find(const ProdTable<void> &t, unsigned char *codes, int 
   const int cap = (int)run_capacity(n);
   const int grid = std::max(1, std::min((cap + 7) / 8, dev_info().sms * 8));
   auto kern = t.prod_of_row ? k_run_key<true> : k_run_key<false>;
-  kern<<<grid, 256, 0, s>>>(t, found, cap, lim, codes, row_nz, runs, rt, sym_sub);
+  kern<<<grid, 256, 0, s>>>(t, found, lim, codes, row_nz, rt, sym_sub);
+  return cudaGetLastError();
+}
+
+// ---- bunches ------------------------------------------------------------------------
+// Rows that no run took (the ends of grid lines above all) still share their
+// patterns with many others, at no fixed distance. They are grouped by pattern
+// alone, with the same hash, table and exact comparison as the runs, and
+// computed by the same programs, each row's B values staged on their own. On
+// the 27-point 128^3 stencil the 65,536 rows at the ends of its lines took 297
+// us in k_sym_map and 305 us in k_num_map, a fifth of the product.
+constexpr int kBunchBits = 19;  // place of a row in its slot; slots take the bits above
+static_assert(kRunSlots <= 1 << (31 - kBunchBits), "slot and place in one int");
+
+template <bool MULTI>
+__global__ void __launch_bounds__(256)
+    k_bunch_key(const ProdTable<void> src, const unsigned char *__restrict__ member, int n,
+                const int *__restrict__ row_nz, const RunTable rt, int *__restrict__ slot_of) {
+  const int lane = threadIdx.x & 31;
+  const int warps = gridDim.x * 8;
+  for (int base = ((blockIdx.x * 256 + threadIdx.x) >> 5) * 32; base < n; base += warps * 32) {
+    const int mine = base + lane;
+    int my_slot = -1;
+    unsigned todo = __ballot_sync(0xffffffffu, mine < n && !member[mine] && row_nz[mine] > 0);
+    while (todo) {
+      const int w = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      const int row = base + w;
+      Operands<void> o;
+      const int lr = prod_row<MULTI>(src, row, o);
+      const int a0 = __ldg(o.arpt + lr), na = __ldg(o.arpt + lr + 1) - a0;
+      if (na > kRunMaxA) continue;
+      unsigned h = 0;
+      int P = 0, cb = 0;
+      bool have = false;
+      for (int c = 0; c < na; c += 32) {
+        const int t = c + lane;
+        int bs = 0, len = 0;
+        if (t < na) {
+          const int k = __ldg(o.acol + a0 + t);
+          bs = __ldg(o.brpt + k);
+          len = __ldg(o.brpt + k + 1) - bs;
+        }
+        // a row of too many products is left before its columns are read
+        int total = len;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
+        P += total;
+        if (total < 0 || total > kRunMaxIp || P > kRunMaxIp) {
+          P = kRunMaxIp + 1;
+          break;
+        }
+        const unsigned some = __ballot_sync(0xffffffffu, len > 0);
+        if (some && !have) {
+          cb = __ldg(o.bcol + __shfl_sync(0xffffffffu, bs, __ffs(some) - 1));
+          have = true;
+        }
+        if (t < na) {
+          h += run_mix((unsigned)len, (unsigned)t + 1u);
+#pragma unroll 4
+          for (int e = 0; e < len; ++e)
+            h += run_mix((unsigned)(__ldg(o.bcol + bs + e) - cb),
+                         (unsigned)(t * 2048 + e) + 0x10000u);
+        }
+      }
+      if (P <= 0 || P > kRunMaxIp) continue;
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) h += __shfl_xor_sync(0xffffffffu, h, d);
+      int prod = 0;
+      if constexpr (MULTI) prod = __ldg(src.prod_of_row + row);
+      h = run_mix(h, (unsigned)na + (unsigned)prod * 0x9e37u);
+      int slot = -1;
+      for (int tries = 0; tries < 16 && slot < 0; ++tries) {
+        const int at = (int)((h + (unsigned)tries) & (kRunSlots - 1));
+        int rep = 0;
+        if (lane == 0) {
+          rep = *(volatile int *)(rt.brep + at);
+          if (rep == 0) rep = atomicCAS(rt.brep + at, 0, row + 1);
+        }
+        rep = __shfl_sync(0xffffffffu, rep, 0);
+        if (rep == 0) {
+          slot = at;
+          break;
+        }
+        Operands<void> o2;
+        const int lr2 = prod_row<MULTI>(src, rep - 1, o2);
+        if constexpr (MULTI)
+          if (__ldg(src.prod_of_row + rep - 1) != prod) continue;
+        const int a2 = __ldg(o2.arpt + lr2);
+        if (__ldg(o2.arpt + lr2 + 1) - a2 != na) continue;
+        bool diff = false, have2 = false;
+        int cb2 = 0;
+        for (int c = 0; c < na && !diff; c += 32) {
+          const int t = c + lane;
+          int bs = 0, len = 0, bs2 = 0, len2 = 0;
+          if (t < na) {
+            const int k = __ldg(o.acol + a0 + t), k2 = __ldg(o2.acol + a2 + t);
+            bs = __ldg(o.brpt + k);
+            len = __ldg(o.brpt + k + 1) - bs;
+            bs2 = __ldg(o2.brpt + k2);
+            len2 = __ldg(o2.brpt + k2 + 1) - bs2;
+            diff = len != len2;
+          }
+          const unsigned some = __ballot_sync(0xffffffffu, len2 > 0);
+          if (some && !have2) {
+            cb2 = __ldg(o2.bcol + __shfl_sync(0xffffffffu, bs2, __ffs(some) - 1));
+            have2 = true;
+          }
+          if (!diff) {
+#pragma unroll 4
+            for (int e = 0; e < len; ++e)
+              diff |= __ldg(o.bcol + bs + e) - cb != __ldg(o2.bcol + bs2 + e) - cb2;
+          }
+          diff = __any_sync(0xffffffffu, diff);
+        }
+        if (!diff) slot = at;
+      }
+      int place = 0;
+      if (slot >= 0) {
+        if (lane == 0) place = atomicAdd(rt.bcount + slot, 1);
+        place = __shfl_sync(0xffffffffu, place, 0);
+      }
+      if (lane == w && slot >= 0 && place < (1 << kBunchBits)) my_slot = slot << kBunchBits | place;
+    }
+    if (mine < n) slot_of[mine] = my_slot;
+  }
+}
+
+// Used slots become bunches, in slot order; one block, kRunSlots / 1024 slots a thread.
+__global__ void __launch_bounds__(1024) k_bunch_plan(const RunTable rt) {
+  constexpr int kPer = kRunSlots / 1024;
+  __shared__ int s_rows[32], s_num[32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  int c[kPer], rows = 0, num = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    c[i] = min(rt.bcount[t * kPer + i], 1 << kBunchBits);
+    rows += c[i];
+    num += c[i] > 0;
+  }
+  const int own_rows = rows, own_num = num;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, rows, d), b = __shfl_up_sync(0xffffffffu, num, d);
+    if (lane >= d) {
+      rows += a;
+      num += b;
+    }
+  }
+  if (lane == 31) {
+    s_rows[warp] = rows;
+    s_num[warp] = num;
+  }
+  __syncthreads();
+  for (int w = 0; w < warp; ++w) {
+    rows += s_rows[w];
+    num += s_num[w];
+  }
+  if (t == 1023) rt.head->nbunch = num;
+  int place = rows - own_rows, b = num - own_num;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    if (c[i] == 0) continue;
+    const int slot = t * kPer + i;
+    rt.bslot[slot] = place;
+    rt.brow[b] = rt.brep[slot] - 1;
+    rt.brows[b] = c[i];
+    rt.bplace[b] = place;
+    place += c[i];
+    ++b;
+  }
+}
+
+__global__ void __launch_bounds__(256)
+    k_bunch_list(const int *__restrict__ slot_of, int n, const RunTable rt, const BinLimits lim,
+                 unsigned char *__restrict__ member, int *__restrict__ row_nz,
+                 int *__restrict__ list, int *__restrict__ sym_sub) {
+  __shared__ int hist[kSymBins];
+  if (threadIdx.x < kSymBins) hist[threadIdx.x] = 0;
+  __syncthreads();
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+    const int v = slot_of[i];
+    if (v < 0) continue;
+    list[rt.bslot[v >> kBunchBits] + (v & ((1 << kBunchBits) - 1))] = i;
+    member[i] = 1;
+    const int ub = row_nz[i];
+    if (ub > 0) atomicAdd(&hist[sym_bin(ub, lim)], 1);
+    row_nz[i] = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x < kSymBins && hist[threadIdx.x])
+    atomicAdd(&sym_sub[threadIdx.x], hist[threadIdx.x]);
+}
+
+cudaError_t launch_bunch_find(const ProdTable<void> &t, unsigned char *member, int n,
+                              const BinLimits &lim, int *row_nz, const RunTable &rt, int *slot,
+                              int *list, int *sym_sub, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  const int grid = std::min((n + 255) / 256, dev_info().sms * 8);
+  auto kern = t.prod_of_row ? k_bunch_key<true> : k_bunch_key<false>;
+  kern<<<grid, 256, 0, s>>>(t, member, n, row_nz, rt, slot);
+  k_bunch_plan<<<1, 1024, 0, s>>>(rt);
+  k_bunch_list<<<grid, 256, 0, s>>>(slot, n, rt, lim, member, row_nz, list, sym_sub);
   return cudaGetLastError();
 }
 
@@ -439,12 +648,18 @@ __host__ __device__ constexpr long long run_tile(int rows, int n, int na, int vs
   return run_out(rows, n) + (long long)rows * run_arow(na, vsz) + 16;
 }
 
-// One block a program.
+// A bunch's rows are staged one by one: their B values in walk order, a row's
+// A values, and where each of its B rows starts.
+__host__ __device__ constexpr int bunch_row(int n, int na, int p, int vsz) {
+  return (n | 1) * 8 + ((na | 1) + (p | 1)) * vsz + 4 * na;
+}
+
+// One block a program: that of run run_of[b], or of bunch b - nprog.
 constexpr int kProgThreads = 512;
 template <bool MULTI>
 __global__ void __launch_bounds__(kProgThreads)
     k_run_prog(const ProdTable<void> src, const RowRun *__restrict__ found,
-               const int *__restrict__ run_of, int vsz, RunProg *__restrict__ progs,
+               const RunTable rt, int nprog, int vsz, RunProg *__restrict__ progs,
                int *__restrict__ err) {
   __shared__ unsigned long long keys[2048];
   __shared__ int tk[kRunMaxA], tbs[kRunMaxA], tlen[kRunMaxA], tpl[kRunMaxA], tpre[kRunMaxA + 1];
@@ -456,8 +671,11 @@ __global__ void __launch_bounds__(kProgThreads)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int W = kProgThreads / 32;
   RunProg &out = progs[blockIdx.x];
-  const RowRun rd = found[run_of[blockIdx.x]];
-  const int sigma = rd.meta >> 2 & 3;
+  const bool bunch = (int)blockIdx.x >= nprog;
+  RowRun rd{0, 0, 0, 0};
+  if (bunch) rd.row0 = rt.brow[blockIdx.x - nprog];
+  else rd = found[rt.run_of[blockIdx.x]];
+  const int sigma = bunch ? 0 : rd.meta >> 2 & 3;
   Operands<void> o;
   const int lr = prod_row<MULTI>(src, rd.row0, o);
   const int a0 = __ldg(o.arpt + lr), na = __ldg(o.arpt + lr + 1) - a0;
@@ -506,6 +724,23 @@ __global__ void __launch_bounds__(kProgThreads)
       out.na = out.p = out.n = 0;
     }
     return;
+  }
+  if (!bunch) {  // runs are listed by program, the classes apart
+    int before = 0;
+    for (int p = tid; p < (int)blockIdx.x; p += kProgThreads) {
+      const int v = rt.slot_of[p];
+      if ((v >> 16) == (P > kRunSmallIp)) before += rt.count[v & 0xffff];
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) before += __shfl_xor_sync(0xffffffffu, before, d);
+    if (lane == 0) s_scan[warp] = before;
+    __syncthreads();
+    if (tid == 0) {
+      int sum = 0;
+      for (int w = 0; w < W; ++w) sum += s_scan[w];
+      rt.first[blockIdx.x] = sum;
+    }
+    __syncthreads();
   }
   // -- the products sorted by (column, walk order)
   const int cb = __ldg(o.bcol + tbs[t0]);
@@ -566,6 +801,17 @@ __global__ void __launch_bounds__(kProgThreads)
   const int warps = large ? RunCfg<1>::WARPS : RunCfg<0>::WARPS;
   if (warp == 0) {
     const int smem = large ? RunCfg<1>::SMEM : RunCfg<0>::SMEM;
+    if (bunch) {
+      const int room = smem - run_fixed(n, P) - 64 - ((P + 15) & ~15) - 2 * (kRunMaxA + 2);
+      int most = min(room / (bunch_row(n, na, P, vsz) + 8), kRunRows);
+      if (most > 32) most &= ~31;
+      if (lane == 0) {
+        s_int[2] = 0;
+        s_int[3] = max(most, 1);
+        s_int[4] = P | 1;
+        s_int[5] = 0;
+      }
+    }
     const int unit = 16 / vsz;
     auto layout = [&](int L, bool write) {  // elements of B; segments in s_int[2]
       const int span = (L - 1) * sigma + 1;
@@ -621,20 +867,22 @@ __global__ void __launch_bounds__(kProgThreads)
       if (fixed > smem) return false;
       return fixed + (long long)layout(L, false) * vsz <= smem;
     };
-    int lo = 1, hi = kRunRows + 1;  // lo fits, hi does not
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (fits(mid)) lo = mid; else hi = mid;
-    }
-    if (lo > 32) lo &= ~31;
-    const int total = layout(lo, true);
-    bool one = true;
-    for (int t = lane; t < na; t += 32) one = one && tpl[t] == tpl[0];
-    one = __all_sync(0xffffffffu, one);
-    if (lane == 0) {
-      s_int[3] = lo;
-      s_int[4] = lo == 1 ? 0 : one ? tpl[0] : -1;
-      s_int[5] = total;
+    if (!bunch) {
+      int lo = 1, hi = kRunRows + 1;  // lo fits, hi does not
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (fits(mid)) lo = mid; else hi = mid;
+      }
+      if (lo > 32) lo &= ~31;
+      const int total = layout(lo, true);
+      bool one = true;
+      for (int t = lane; t < na; t += 32) one = one && tpl[t] == tpl[0];
+      one = __all_sync(0xffffffffu, one);
+      if (lane == 0) {
+        s_int[3] = lo;
+        s_int[4] = lo == 1 ? 0 : one ? tpl[0] : -1;
+        s_int[5] = total;
+      }
     }
   }
   // -- entries by descending product count, dealt to the parts
@@ -684,6 +932,7 @@ __global__ void __launch_bounds__(kProgThreads)
     out.belems = s_int[5];
   }
   for (int i = tid; i < P + 32; i += kProgThreads) out.word[i] = make_uint2(0u, 0u);
+  if (tid <= na) out.before[tid] = (short)tpre[tid];
   __syncthreads();
   for (int i = tid; i < P; i += kProgThreads) {
     const int p = (int)(unsigned)keys[i], q = sq[i];
@@ -693,6 +942,14 @@ __global__ void __launch_bounds__(kProgThreads)
       if (tpre[mid] <= p) lo = mid; else hi = mid;
     }
     while (tpre[lo + 1] <= p) ++lo;
+    if (bunch) {
+      out.term[p] = (unsigned char)lo;
+      out.word[s_w0[ow[q]] + ooff[q] + (i - hstart[q])] =
+          make_uint2((unsigned)(p * vsz),
+                     (unsigned)(lo * vsz) | (unsigned)q << 11 |
+                         (i + 1 == hstart[q + 1] ? 0x80000000u : 0u));
+      continue;
+    }
     const int g = tseg[lo];
     // a place counts from its segment's 16-byte boundary; the copy's start
     // within the boundary is added tile by tile
@@ -706,34 +963,38 @@ __global__ void __launch_bounds__(kProgThreads)
 }
 
 cudaError_t launch_run_progs(const ProdTable<void> &t, const RowRun *found, const RunTable &rt,
-                             int nprog, bool fp32, void *progs, int *err, cudaStream_t s) {
-  if (nprog <= 0) return cudaSuccess;
+                             int nprog, int nbunch, bool fp32, void *progs, int *err,
+                             cudaStream_t s) {
+  if (nprog + nbunch <= 0) return cudaSuccess;
   auto kern = t.prod_of_row ? k_run_prog<true> : k_run_prog<false>;
-  kern<<<nprog, kProgThreads, 0, s>>>(t, found, rt.run_of, fp32 ? 4 : 8,
-                                      static_cast<RunProg *>(progs), err);
+  kern<<<nprog + nbunch, kProgThreads, 0, s>>>(t, found, rt, nprog, fp32 ? 4 : 8,
+                                               static_cast<RunProg *>(progs), err);
   return cudaGetLastError();
 }
 
-// Every run's slot in the table becomes its program; with row_nz its rows get
-// their count there; they are counted as numeric-bin rows that no bin needs
-// (by crpt, what k_perm goes by, when row_nz is null).
+// The list of the runs (small ones from the front of `runs`, large ones from
+// the back), by program; with row_nz their rows get their count there; they
+// are counted as numeric-bin rows that no bin needs (by crpt, what k_perm goes
+// by, when row_nz is null).
 __global__ void __launch_bounds__(256)
-    k_run_counts(RowRun *__restrict__ runs, int small, int large, int cap,
-                 const int *__restrict__ prog_of, const RunProg *__restrict__ progs,
-                 int *__restrict__ row_nz, const int *__restrict__ crpt, const BinLimits lim,
-                 int *__restrict__ num_sub) {
+    k_run_counts(const RowRun *__restrict__ found, int nfound, RowRun *__restrict__ runs, int cap,
+                 const RunTable rt, const RunProg *__restrict__ progs, int *__restrict__ row_nz,
+                 const int *__restrict__ crpt, const BinLimits lim, int *__restrict__ num_sub) {
   __shared__ int hist[kNumBins];
   if (threadIdx.x < kNumBins) hist[threadIdx.x] = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  for (int q = (blockIdx.x * 256 + threadIdx.x) >> 5; q < small + large; q += gridDim.x * 8) {
-    RowRun *r = runs + (q < small ? q : cap - 1 - (q - small));
-    const RowRun rd = *r;
+  for (int q = (blockIdx.x * 256 + threadIdx.x) >> 5; q < nfound; q += gridDim.x * 8) {
+    RowRun rd = found[q];
+    if (rd.prog < 0) continue;
     const int s = rd.meta & 3, len = rd.meta >> 4;
-    const int p = prog_of[rd.prog];
+    const int p = rt.prog_of[rd.prog];
     const int n = progs[p].n;
-    __syncwarp();
-    if (lane == 0) r->prog = p;
+    if (lane == 0) {
+      const int at = rt.first[p] + rd.place;
+      rd.prog = p;
+      runs[rt.slot_of[p] >> 16 ? cap - 1 - at : at] = rd;
+    }
     if (row_nz) {
       if (lane == 0 && n > 0) atomicAdd(&hist[num_bin(n, lim)], len);
       for (int m = lane; m < len; m += 32) row_nz[rd.row0 + s * m] = n;
@@ -750,14 +1011,73 @@ __global__ void __launch_bounds__(256)
     atomicAdd(&num_sub[threadIdx.x], hist[threadIdx.x]);
 }
 
-cudaError_t launch_run_counts(RowRun *runs, const int (&nruns)[2], int cap, const RunTable &rt,
-                              const void *progs, int *row_nz, const int *crpt,
+cudaError_t launch_run_counts(const RowRun *found, int nfound, RowRun *runs, int cap,
+                              const RunTable &rt, const void *progs, int *row_nz, const int *crpt,
                               const BinLimits &lim, int *num_sub, cudaStream_t s) {
-  const int all = nruns[0] + nruns[1];
-  if (all <= 0) return cudaSuccess;
-  const int grid = std::min((all + 7) / 8, dev_info().sms * 8);
-  k_run_counts<<<grid, 256, 0, s>>>(runs, nruns[0], nruns[1], cap, rt.prog_of,
+  if (nfound <= 0) return cudaSuccess;
+  const int grid = std::min((nfound + 7) / 8, dev_info().sms * 8);
+  k_run_counts<<<grid, 256, 0, s>>>(found, nfound, runs, cap, rt,
                                     static_cast<const RunProg *>(progs), row_nz, crpt, lim, num_sub);
+  return cudaGetLastError();
+}
+
+// The same for the rows of the bunches; blockIdx.y is the bunch. The first
+// block also adds up the tiles of every bunch, by class.
+__global__ void __launch_bounds__(256)
+    k_bunch_counts(const RunTable rt, int nprog, const int *__restrict__ list,
+                   const RunProg *__restrict__ progs, int *__restrict__ row_nz,
+                   const int *__restrict__ crpt, const BinLimits lim, int *__restrict__ num_sub) {
+  const int b = blockIdx.y;
+  if (blockIdx.x == 0 && b == 0) {
+    __shared__ int part[2][256];
+    const int nb = gridDim.y, per = (nb + 255) / 256, first = (int)threadIdx.x * per;
+    int sum[2] = {0, 0};
+    auto tiles = [&](int i, int c) {
+      const RunProg &pg = progs[nprog + i];
+      return pg.n > 0 && (pg.p > kRunSmallIp) == (c == 1) ? (rt.brows[i] + pg.rows - 1) / pg.rows : 0;
+    };
+    for (int i = first; i < min(first + per, nb); ++i)
+      for (int c = 0; c < 2; ++c) sum[c] += tiles(i, c);
+    for (int c = 0; c < 2; ++c) part[c][threadIdx.x] = sum[c];
+    __syncthreads();
+    for (int c = 0; c < 2; ++c) {
+      int at = 0;
+      for (int i = 0; i < (int)threadIdx.x; ++i) at += part[c][i];
+      for (int i = first; i < min(first + per, nb); ++i) {
+        rt.btiles[c][i] = at;
+        at += tiles(i, c);
+      }
+      if (first < nb && first + per >= nb) rt.btiles[c][nb] = at;
+    }
+  }
+  const int n = progs[nprog + b].n, rows = rt.brows[b];
+  const int *rl = list + rt.bplace[b];
+  int mine = 0;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < rows; i += gridDim.x * 256) {
+    if (row_nz) {
+      row_nz[rl[i]] = n;
+    } else {
+      const int v = crpt[rl[i] + 1] - crpt[rl[i]];
+      if (v == n) ++mine;
+      else if (v > 0) atomicAdd(&num_sub[num_bin(v, lim)], 1);
+    }
+  }
+  if (row_nz) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && n > 0) atomicAdd(&num_sub[num_bin(n, lim)], rows);
+  } else {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, d);
+    if ((threadIdx.x & 31) == 0 && mine && n > 0) atomicAdd(&num_sub[num_bin(n, lim)], mine);
+  }
+}
+
+cudaError_t launch_bunch_counts(const RunTable &rt, int nprog, int nbunch, const int *list,
+                                const void *progs, int *row_nz, const int *crpt,
+                                const BinLimits &lim, int *num_sub, cudaStream_t s) {
+  if (nbunch <= 0) return cudaSuccess;
+  k_bunch_counts<<<dim3(8, nbunch), 256, 0, s>>>(rt, nprog, list,
+                                                  static_cast<const RunProg *>(progs), row_nz,
+                                                  crpt, lim, num_sub);
   return cudaGetLastError();
 }
 
@@ -773,18 +1093,24 @@ cudaError_t launch_run_counts(RowRun *runs, const int (&nruns)[2], int cap, cons
 // boundary at or before its first value; how far into it that value lies
 // changes from tile to tile and is added to the program's words. A staged
 // value is read where it is used, a lane per row: odd row lengths spread the
-// lanes over all banks. One warp more only looks up what the next tile needs
-// (its run, the places of its rows) and starts its copies as soon as the
-// others have computed the tile before, while they write that tile out; with
-// the look-ups left to the computing warps they took as long as the sums
-// (5,700 of 14,200 cycles a tile of the 27-point stencil). Where the rows of C
+// lanes over all banks. One or two warps more only look up what tiles need
+// (their run, the places of their rows), each for runs of its own, and start
+// the copies of the next tile as soon as the others have computed the one
+// before, while they write it out. With the look-ups left to the computing
+// warps they took as long as the sums (5,700 of 14,200 cycles a tile of the
+// 27-point stencil); with one warp for them the chain of five dependent loads a
+// run bound the tiles of few products (7-point 149 x 131 x 97: 377 us, 311 with
+// two; a second warp gains nothing where a run has several large tiles). Runs
+// are listed by program, so that a block seldom changes it: the parts of
+// another program lie elsewhere, and its tile has to wait for the last one to
+// be written out. Where the rows of C
 // lie one after the other (s = 1, an odd count) their values leave by one bulk
 // copy too.
 //
 // What bounds it: two 8-byte shared-memory reads and a multiply and add per
 // product, four wavefronts for 32 products, against about 22 and a barrier a
 // step for the entry-map kernel's read-modify-write of a value slot.
-constexpr int kCopyWait = 1 << 20;  // polls before a wait for a copy gives up
+constexpr int kCopyWait = 1 << 20;  // polls before a wait gives up
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
@@ -868,6 +1194,59 @@ struct RunSmem {
   }
 };
 
+// Words [w0, w1) of a program for one row: al its A values, b_of a word's B
+// value, ol the row's entries of C.
+template <typename VT, bool COMP, typename F>
+__device__ __forceinline__ void run_walk(const uint2 *prog, int w0, int w1, const char *al,
+                                         bool pair, bool write, double *ol, F &&b_of) {
+  auto a_of = [&](uint2 w) { return *reinterpret_cast<const VT *>(al + (w.y & 0x7ffu)); };
+  auto rank = [](unsigned y) { return y >> 11 & 0x7ffu; };
+  if (!COMP || !pair) {
+    double acc = 0.0;
+    auto step = [&](unsigned y, VT a, VT b) {
+      acc = __dadd_rn(acc, __dmul_rn((double)a, (double)b));
+      if ((int)y < 0) {
+        if (write) ol[rank(y)] = acc;
+        acc = 0.0;
+      }
+    };
+    int p = w0;
+    for (; p + 4 <= w1; p += 4) {
+      const uint4 u = *reinterpret_cast<const uint4 *>(prog + p);
+      const uint4 v = *reinterpret_cast<const uint4 *>(prog + p + 2);
+      const uint2 q0 = make_uint2(u.x, u.y), q1 = make_uint2(u.z, u.w);
+      const uint2 q2 = make_uint2(v.x, v.y), q3 = make_uint2(v.z, v.w);
+      const VT x0 = a_of(q0), x1 = a_of(q1), x2 = a_of(q2), x3 = a_of(q3);
+      const VT y0 = b_of(q0), y1 = b_of(q1), y2 = b_of(q2), y3 = b_of(q3);
+      step(u.y, x0, y0);
+      step(u.w, x1, y1);
+      step(v.y, x2, y2);
+      step(v.w, x3, y3);
+    }
+    for (; p < w1; ++p) {
+      const uint2 w = prog[p];
+      step(w.y, a_of(w), b_of(w));
+    }
+  } else {
+    // error-free fp32 pairs, started from the entry's first product
+    bool fresh = true;
+    float2 sc = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int p = w0; p < w1; ++p) {
+      const uint2 w = prog[p];
+      const float a = (float)a_of(w), b = (float)b_of(w);
+      if (fresh) {
+        const float ph = __fmul_rn(a, b);
+        sc = make_float2(ph, __fmaf_rn(a, b, -ph));
+      } else {
+        comp_add(sc, a, b);
+      }
+      fresh = (int)w.y < 0;
+      if (fresh && write) ol[rank(w.y)] = (double)sc.x + (double)sc.y;
+    }
+  }
+}
+
 // What the look-up warp leaves for a tile.
 struct RunTile {
   int prog;   // -1: no more tiles
@@ -881,7 +1260,7 @@ struct RunTile {
 };
 
 template <int CLASS, typename VT, bool COMP, bool MULTI>
-__global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32 + 32, RunCfg<CLASS>::MINB)
+__global__ void __launch_bounds__((RunCfg<CLASS>::WARPS + RunCfg<CLASS>::LOOK) * 32, RunCfg<CLASS>::MINB)
     k_num_run(const ProdTable<VT> src, const RowRun *__restrict__ runs, int nruns,
               const RunProg *__restrict__ progs, const int *__restrict__ crpt,
               int *__restrict__ ccol, double *__restrict__ cval, int *__restrict__ err,
@@ -891,9 +1270,10 @@ __global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32 + 32, RunCfg<CLASS>:
   __shared__ __align__(8) unsigned long long s_full, s_done, s_free[2];
   __shared__ RunTile s_tile[2];
   __shared__ unsigned char held[kRunMaxA];  // the leads that the words hold
-  __shared__ int s_lost;
+  __shared__ int s_lost, s_tiles, s_ended;  // tiles announced, look-up warps that have ended
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {
+    s_tiles = s_ended = 0;
     mbar_init(&s_full, 1);        // a tile's data and values are there
     mbar_init(&s_done, 1);        // it is computed: the next one's values may come
     mbar_init(&s_free[0], WARPS); // it is written out: its data may be replaced
@@ -903,9 +1283,9 @@ __global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32 + 32, RunCfg<CLASS>:
   }
   __syncthreads();
 
-  if (warp == WARPS) {
-    // -- the look-up warp
-    int t = 0, cur = -1, next = 0;
+  if (warp >= WARPS) {
+    // -- the look-up warps
+    int next = 0;
     bool lost = false;
     int max_deg = 0, redo = 0;
     if (lane == 0) next = atomicAdd(ticket, 1);
@@ -944,10 +1324,9 @@ __global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32 + 32, RunCfg<CLASS>:
         if (na <= comp.nmax) max_deg = max(max_deg, na);
         else redo += len;
       }
-      for (int r0 = 0; r0 < len && !lost; r0 += L, ++t) {
+      for (int r0 = 0; r0 < len && !lost; r0 += L) {
         const int cnt = min(L, len - r0);
         const int adv = sigma * r0, reach = sigma * (r0 + cnt - 1) + 1;
-        RunTile &tile = s_tile[t & 1];
         int b0[kPer], b1[kPer];
 #pragma unroll
         for (int i = 0; i < kPer; ++i)
@@ -978,6 +1357,11 @@ __global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32 + 32, RunCfg<CLASS>:
           }
         }
         in_line = __all_sync(0xffffffffu, in_line);
+        // everything is looked up: this is the block's next tile
+        int t = 0;
+        if (lane == 0) t = atomicAdd(&s_tiles, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        RunTile &tile = s_tile[t & 1];
         if (t >= 2 && !mbar_wait(&s_free[t & 1], (unsigned)((t >> 1) - 1) & 1u)) lost = true;
         unsigned bytes = 0;
 #pragma unroll
@@ -1007,15 +1391,15 @@ __global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32 + 32, RunCfg<CLASS>:
         }
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, d);
-        // another program has its parts elsewhere: the last tile must be out
         if (t >= 1) {
-          const bool came = rd.prog == cur ? mbar_wait(&s_done, (unsigned)(t - 1) & 1u)
-                                           : mbar_wait(&s_free[(t - 1) & 1], (unsigned)((t - 1) >> 1) & 1u);
-          lost = lost || !came;
+          if (!mbar_wait(&s_done, (unsigned)(t - 1) & 1u)) lost = true;
+          // another program has its parts elsewhere: the last tile must be out
+          if (!lost && *(volatile int *)&s_tile[(t - 1) & 1].prog != rd.prog &&
+              !mbar_wait(&s_free[(t - 1) & 1], (unsigned)((t - 1) >> 1) & 1u))
+            lost = true;
         }
         lost = __any_sync(0xffffffffu, lost);
         if (lost) break;
-        cur = rd.prog;
         __syncwarp();
         if (lane == 0) mbar_expect(&s_full, bytes);
         __syncwarp();
@@ -1040,16 +1424,22 @@ __global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32 + 32, RunCfg<CLASS>:
       }
     }
     // no more tiles: the computing warps end on a tile without a program, which
-    // may be announced once the last one's values have arrived (two arrivals in
-    // one phase of s_full are one too many)
-    if (!lost && t >= 1 && !mbar_wait(&s_done, (unsigned)(t - 1) & 1u)) lost = true;
-    if (!lost && t >= 2 && !mbar_wait(&s_free[t & 1], (unsigned)((t >> 1) - 1) & 1u)) lost = true;
+    // the last look-up warp announces once the last tile's values have arrived
+    // (two arrivals in one phase of s_full are one too many)
+    int ended = 0;
+    if (lane == 0) ended = atomicAdd(&s_ended, 1);
+    ended = __shfl_sync(0xffffffffu, ended, 0);
+    const int t = *(volatile int *)&s_tiles;
+    const bool last = ended == RunCfg<CLASS>::LOOK - 1;
+    if (last && !lost && t >= 1 && !mbar_wait(&s_done, (unsigned)(t - 1) & 1u)) lost = true;
+    if (last && !lost && t >= 2 && !mbar_wait(&s_free[t & 1], (unsigned)((t >> 1) - 1) & 1u))
+      lost = true;
     if (lost) {
       if (lane == 0) {
         atomicExch(&s_lost, 1);
         atomicOr(err, ERR_WAIT);
       }
-    } else if (lane == 0) {
+    } else if (last && lane == 0) {
       s_tile[t & 1].prog = -1;
       mbar_expect(&s_full, 0);
     }
@@ -1122,59 +1512,11 @@ __global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32 + 32, RunCfg<CLASS>:
       double *ol = out0 + (size_t)ll * npad;
       const char *bl = reinterpret_cast<const char *>(sm.bs + (pstep > 0 ? pstep : 0) * ll);
       const int lb = ll * (int)sizeof(VT);
-      const uint2 *prog = sm.prog;
-      auto a_of = [&](uint2 w) { return *reinterpret_cast<const VT *>(al + (w.y & 0x7ffu)); };
-      auto rank = [](unsigned y) { return y >> 11 & 0x7ffu; };
-      auto walk = [&](auto b_of) {
-        if (!COMP || !pair) {
-          double acc = 0.0;
-          auto step = [&](unsigned y, VT a, VT b) {
-            acc = __dadd_rn(acc, __dmul_rn((double)a, (double)b));
-            if ((int)y < 0) {
-              if (write) ol[rank(y)] = acc;
-              acc = 0.0;
-            }
-          };
-          int p = w0;
-          for (; p + 4 <= w1; p += 4) {
-            const uint4 u = *reinterpret_cast<const uint4 *>(prog + p);
-            const uint4 v = *reinterpret_cast<const uint4 *>(prog + p + 2);
-            const uint2 q0 = make_uint2(u.x, u.y), q1 = make_uint2(u.z, u.w);
-            const uint2 q2 = make_uint2(v.x, v.y), q3 = make_uint2(v.z, v.w);
-            const VT x0 = a_of(q0), x1 = a_of(q1), x2 = a_of(q2), x3 = a_of(q3);
-            const VT y0 = b_of(q0), y1 = b_of(q1), y2 = b_of(q2), y3 = b_of(q3);
-            step(u.y, x0, y0);
-            step(u.w, x1, y1);
-            step(v.y, x2, y2);
-            step(v.w, x3, y3);
-          }
-          for (; p < w1; ++p) {
-            const uint2 w = prog[p];
-            step(w.y, a_of(w), b_of(w));
-          }
-        } else {
-          // error-free fp32 pairs, started from the entry's first product
-          bool fresh = true;
-          float2 sc = make_float2(0.f, 0.f);
-#pragma unroll 4
-          for (int p = w0; p < w1; ++p) {
-            const uint2 w = prog[p];
-            const float a = (float)a_of(w), b = (float)b_of(w);
-            if (fresh) {
-              const float ph = __fmul_rn(a, b);
-              sc = make_float2(ph, __fmaf_rn(a, b, -ph));
-            } else {
-              comp_add(sc, a, b);
-            }
-            fresh = (int)w.y < 0;
-            if (fresh && write) ol[rank(w.y)] = (double)sc.x + (double)sc.y;
-          }
-        }
-      };
       if (pstep >= 0)
-        walk([&](uint2 w) { return *reinterpret_cast<const VT *>(bl + w.x); });
+        run_walk<VT, COMP>(sm.prog, w0, w1, al, pair, write, ol,
+                           [&](uint2 w) { return *reinterpret_cast<const VT *>(bl + w.x); });
       else
-        walk([&](uint2 w) {
+        run_walk<VT, COMP>(sm.prog, w0, w1, al, pair, write, ol, [&](uint2 w) {
           return *reinterpret_cast<const VT *>(bl + (w.x & 0x1ffffu) + (w.x >> 17) * lb);
         });
     }
@@ -1224,7 +1566,7 @@ static cudaError_t run_num_run(const ProdTable<VT> &t, const RowRun *runs, int n
   if (nruns <= 0) return cudaSuccess;
   using C = RunCfg<CLASS>;
   auto kern = t.prod_of_row ? k_num_run<CLASS, VT, COMP, true> : k_num_run<CLASS, VT, COMP, false>;
-  const int threads = C::WARPS * 32 + 32;
+  const int threads = (C::WARPS + C::LOOK) * 32;
   const int grid = persistent_grid((const void *)kern, threads, C::SMEM, nruns, 1);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
   kern<<<grid, threads, C::SMEM, s>>>(t, runs, nruns, static_cast<const RunProg *>(progs),
@@ -1256,6 +1598,156 @@ cudaError_t launch_numeric_comp_run(const ProdTable<float> &t, const RowRun *run
                                     int *max_deg, int *err, int *ticket, cudaStream_t s) {
   return run_num_runs<float, true>(t, runs, nruns, cap, progs, crpt, ccol, cval, err,
                                    CompArgs{nmax, redo, max_deg}, ticket, s);
+}
+
+// ---- numeric phase of the bunches --------------------------------------------------
+// As k_num_run, but a tile's rows lie anywhere: each row's B values are staged
+// in walk order (product p at place p), a warp a row. Few rows come here (those
+// at the ends of grid lines); 14 rows of a 27-point stencil fill a block's
+// shared memory. Bound by the look-ups of a tile's rows, which two to four
+// blocks an SM overlap.
+template <int CLASS, typename VT, bool COMP, bool MULTI>
+__global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32, RunCfg<CLASS>::MINB)
+    k_num_bunch(const ProdTable<VT> src, const RunTable rt, int nprog, int nbunch,
+                const int *__restrict__ list, const RunProg *__restrict__ progs,
+                const int *__restrict__ crpt, int *__restrict__ ccol, double *__restrict__ cval,
+                int *__restrict__ err, CompArgs comp, int *__restrict__ ticket) {
+  constexpr int WARPS = RunCfg<CLASS>::WARPS, THREADS = WARPS * 32;
+  extern __shared__ __align__(16) unsigned char smem_bunch[];
+  __shared__ int s_next, s_bunch;
+  __shared__ int s_c0[kRunRows], s_cb[kRunRows];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int *tiles = rt.btiles[CLASS];  // before each bunch
+  const int all = __ldg(tiles + nbunch);
+  int cur = -1, redo = 0, max_deg = 0;
+  for (;;) {
+    __syncthreads();  // the last tile is written out
+    if (tid == 0) s_next = atomicAdd(ticket, 1);
+    __syncthreads();
+    const int at = s_next;
+    if (at >= all) break;
+    for (int i = tid; i < nbunch; i += THREADS)
+      if (__ldg(tiles + i) <= at && at < __ldg(tiles + i + 1)) s_bunch = i;
+    __syncthreads();
+    const int b = s_bunch;
+    const RunProg &pg = progs[nprog + b];
+    const int na = pg.na, P = pg.p, n = pg.n, L = pg.rows, parts = pg.parts;
+    const int r0 = (at - __ldg(tiles + b)) * L, cnt = min(L, rt.brows[b] - r0);
+    const int *rl = list + rt.bplace[b] + r0;
+    uint2 *prog = reinterpret_cast<uint2 *>(smem_bunch);
+    int *rel = reinterpret_cast<int *>(prog + P + 32);
+    double *out = reinterpret_cast<double *>(smem_bunch + run_fixed(n, P));
+    VT *As = reinterpret_cast<VT *>(out + (size_t)L * (n | 1));
+    VT *Bs = As + (size_t)L * (na | 1);
+    int *from = reinterpret_cast<int *>(Bs + (size_t)L * (P | 1));  // B row start - its place
+    unsigned char *term = reinterpret_cast<unsigned char *>(from + (size_t)L * na);
+    short *before = reinterpret_cast<short *>(term + ((P + 15) & ~15));
+    if (b != cur) {
+      cur = b;
+      for (int i = tid; i < P + 32; i += THREADS) prog[i] = pg.word[i];
+      for (int i = tid; i < n; i += THREADS) rel[i] = pg.rel[i];
+      for (int i = tid; i < P; i += THREADS) term[i] = pg.term[i];
+      for (int i = tid; i <= na; i += THREADS) before[i] = pg.before[i];
+    }
+    const bool pair = COMP && na <= comp.nmax;
+    if (COMP && tid == 0) {
+      if (pair) max_deg = max(max_deg, na);
+      else redo += cnt;
+    }
+    __syncthreads();
+    Operands<VT> op;  // every row of a bunch is of one product
+    prod_row<MULTI>(src, rl[0], op);
+    const int first = MULTI ? __ldg(src.row_off + __ldg(src.prod_of_row + rl[0])) : 0;
+    for (int l = warp; l < cnt; l += WARPS) {
+      const int row = rl[l];
+      const int a0 = __ldg(op.arpt + row - first);
+      for (int t = lane; t < na; t += 32) {
+        const int b0 = __ldg(op.brpt + __ldg(op.acol + a0 + t));
+        from[l * na + t] = b0 - before[t];
+        As[l * (na | 1) + t] = __ldg(op.aval + a0 + t);
+        if (t == pg.t0) s_cb[l] = __ldg(op.bcol + b0);
+      }
+      if (lane == 0) {
+        const int c0 = __ldg(crpt + row);
+        const bool fits = __ldg(crpt + row + 1) - c0 == n;
+        if (!fits) atomicOr(err, ERR_COUNT);
+        s_c0[l] = fits ? c0 : -1;
+      }
+      __syncwarp();
+      VT *bl = Bs + (size_t)l * (P | 1);
+#pragma unroll 4
+      for (int p = lane; p < P; p += 32)
+        __pipeline_memcpy_async(bl + p, op.bval + from[l * na + term[p]] + p, sizeof(VT));
+    }
+    __pipeline_commit();
+    __pipeline_wait_prior(0);
+    __syncthreads();
+    const int rg = warp / parts, part = warp - rg * parts;
+    if (rg * 32 < cnt && rg < (L + 31) / 32) {
+      const int l = rg * 32 + lane, ll = min(l, cnt - 1);
+      const char *bl = reinterpret_cast<const char *>(Bs + (size_t)ll * (P | 1));
+      run_walk<VT, COMP>(prog, pg.w0[part], pg.w1[part],
+                         reinterpret_cast<const char *>(As + ll * (na | 1)), pair, l < cnt,
+                         out + (size_t)ll * (n | 1),
+                         [&](uint2 w) { return *reinterpret_cast<const VT *>(bl + w.x); });
+    }
+    __syncthreads();
+    const int gw = n <= 4 ? 4 : n <= 8 ? 8 : n <= 16 ? 16 : 32;
+    for (int l = tid / gw; l < cnt; l += THREADS / gw) {
+      const int c0 = s_c0[l], cb = s_cb[l];
+      if (c0 < 0) continue;
+      for (int q = tid & (gw - 1); q < n; q += gw) {
+        __stcs(ccol + c0 + q, rel[q] + cb);
+        __stcs(cval + c0 + q, out[(size_t)l * (n | 1) + q]);
+      }
+    }
+  }
+  if (COMP && tid == 0) {
+    if (max_deg) atomicMax(comp.max_deg, max_deg);
+    if (redo) atomicAdd(comp.redo, redo);
+  }
+}
+
+template <int CLASS, typename VT, bool COMP>
+static cudaError_t run_num_bunch(const ProdTable<VT> &t, const RunTable &rt, int nprog, int nbunch,
+                                 const int *list, const void *progs, const int *crpt, int *ccol,
+                                 double *cval, int *err, CompArgs comp, int *ticket,
+                                 cudaStream_t s) {
+  using C = RunCfg<CLASS>;
+  auto kern = t.prod_of_row ? k_num_bunch<CLASS, VT, COMP, true> : k_num_bunch<CLASS, VT, COMP, false>;
+  // how many tiles there are is known on the device only
+  const int grid = persistent_grid((const void *)kern, C::WARPS * 32, C::SMEM, INT32_MAX, 1);
+  if (grid <= 0) return cudaErrorInvalidConfiguration;
+  kern<<<grid, C::WARPS * 32, C::SMEM, s>>>(t, rt, nprog, nbunch, list,
+                                            static_cast<const RunProg *>(progs), crpt, ccol, cval,
+                                            err, comp, ticket);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_numeric_bunch(const ProdTable<double> &t, const RunTable &rt, int nprog,
+                                 int nbunch, const int *list, const void *progs, const int *crpt,
+                                 int *ccol, double *cval, int *err, int *ticket, cudaStream_t s) {
+  if (nbunch <= 0) return cudaSuccess;
+  const CompArgs none{0, nullptr, nullptr};
+  cudaError_t e = run_num_bunch<1, double, false>(t, rt, nprog, nbunch, list, progs, crpt, ccol,
+                                                  cval, err, none, ticket + 1, s);
+  if (e != cudaSuccess) return e;
+  return run_num_bunch<0, double, false>(t, rt, nprog, nbunch, list, progs, crpt, ccol, cval, err,
+                                         none, ticket, s);
+}
+
+cudaError_t launch_numeric_comp_bunch(const ProdTable<float> &t, const RunTable &rt, int nprog,
+                                      int nbunch, const int *list, const void *progs,
+                                      const int *crpt, int *ccol, double *cval, int nmax,
+                                      int *redo, int *max_deg, int *err, int *ticket,
+                                      cudaStream_t s) {
+  if (nbunch <= 0) return cudaSuccess;
+  const CompArgs comp{nmax, redo, max_deg};
+  cudaError_t e = run_num_bunch<1, float, true>(t, rt, nprog, nbunch, list, progs, crpt, ccol,
+                                                cval, err, comp, ticket + 1, s);
+  if (e != cudaSuccess) return e;
+  return run_num_bunch<0, float, true>(t, rt, nprog, nbunch, list, progs, crpt, ccol, cval, err,
+                                       comp, ticket, s);
 }
 
 }  // namespace nspb

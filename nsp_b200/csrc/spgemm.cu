@@ -201,8 +201,10 @@ size_t Call::scratch_bytes() {
   off_row_nz = 0;
   off_perm = align256(off_row_nz + (nn + 1) * 4);
   off_slots = align256(off_perm + nn * 4);
-  off_counters = align256(off_slots + 2 * kRunSlots * 4);
-  off_tiles = align256(off_counters + sizeof(DevCounters) + kRunSlots * 4);
+  off_counters = off_slots;
+  if (allow_runs) off_counters = align256(off_slots + kRunTableRest * (kRunSlots + 64) * 4);
+  off_tiles = align256(off_counters + counter_bytes() +
+                       (allow_runs ? kRunTableZeroed * kRunSlots * 4 : 0));
   const size_t tiles = (size_t)scan_tiles(n);
   ws_bytes = align256(off_tiles + tiles * 8);
   return ws_bytes;
@@ -222,10 +224,18 @@ int Call::alloc_scratch() {
   perm = reinterpret_cast<int *>(ws + off_perm);
   ctr = reinterpret_cast<DevCounters *>(ws + off_counters);
   tile_state = reinterpret_cast<unsigned long long *>(ws + off_tiles);
-  rtab.head = &ctr->run;
-  rtab.rep = reinterpret_cast<int *>(ctr + 1);
-  rtab.prog_of = reinterpret_cast<int *>(ws + off_slots);
-  rtab.run_of = rtab.prog_of + kRunSlots;
+  if (allow_runs) {
+    rtab.head = &ctr->run;
+    rtab.rep = reinterpret_cast<int *>(ctr + 1);
+    rtab.prog_of = reinterpret_cast<int *>(ws + off_slots);
+    rtab.brep = rtab.rep + kRunSlots;
+    rtab.bcount = rtab.brep + kRunSlots;
+    rtab.count = rtab.bcount + kRunSlots;
+    int *rest = rtab.prog_of;
+    for (int **p : {&rtab.run_of, &rtab.slot_of, &rtab.first, &rtab.bslot, &rtab.brow, &rtab.brows, &rtab.bplace, &rtab.btiles[0],
+                    &rtab.btiles[1]})
+      *p = rest += kRunSlots + 64;
+  }
   // counters, pattern table and scan tile states are contiguous: one memset clears them
   cudaError_t e = cudaMemsetAsync(ws + off_counters, 0, ws_bytes - off_counters, s);
   if (e != cudaSuccess) return cuda_fail(e);
@@ -263,7 +273,7 @@ cudaError_t Call::order_block_bins(const int *key, int kind, const int *counts, 
 int Call::fetch_counters() {
   HostStage *hs = stage ? stage : host_stage();
   if (!hs) return NSPB_ERR_ALLOC;
-  cudaError_t e = cudaMemcpyAsync(&hs->c, ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost, s);
+  cudaError_t e = cudaMemcpyAsync(&hs->c, ctr, counter_bytes(), cudaMemcpyDeviceToHost, s);
   if (e != cudaSuccess) return cuda_fail(e);
   e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_fail(e);
@@ -289,28 +299,35 @@ static BinOffsets offsets_of(const int *counts, int nb, int *nonempty, int *tota
 
 // Row runs are looked for when the caller leaves the choice of the row kernels
 // to the library and A's rows are short enough on average for runs to hold
-// most of them. The search costs a pass over B's columns and six launches, so a
-// product of fewer than about 24 million intermediate products (A's entries
-// times B's mean row) does without, unless row_kernel is 8. Measured, runs
-// against none: 27-point 40^3 (42 M) 379 vs 519 us, 32^3 (21 M) 288 vs 317, 24^3
-// (8.5 M) 268 vs 222, R (A P) of 60^3 (11 M) 401 vs 360.
+// most of them. The search and the programs cost a chain of ten small launches,
+// so small products do without, unless row_kernel is 8: those of fewer than
+// about 24 million intermediate products (A's entries times B's mean row), or 6
+// million where B's rows are so short that the row-group kernels leave most
+// lanes idle. Measured, runs against none: 27-point 32^3 (21 M) 289 vs 321 us,
+// 24^3 (8.5 M) 282 vs 222, R (A P) of 60^3 (11 M) 396 vs 357; 7-point 64 x 50 x 50
+// (7.6 M) 244 vs 284, 32^3 (1.5 M) 214 vs 167, A P of 40^3 (7.4 M) 303 vs 332.
 bool Call::runs_wanted() const {
   if (!allow_runs || family() != 0 || (opts.row_kernel & kNoRowTemplates)) return false;
   if (n < 2 * kRunMin || a_nnz > (int64_t)kRunMaxA * n || (table && !info.bdel)) return false;
   if ((opts.row_kernel & 0xff) == 8) return true;
-  return info.brows > 0 && (double)a_nnz * (double)b_nnz >= 24e6 * (double)info.brows;
+  if (info.brows <= 0) return false;
+  const double mean = (double)b_nnz / (double)info.brows;
+  return (double)a_nnz * mean >= (mean < 8.0 ? 6e6 : 24e6);
 }
 
 int Call::alloc_runs() {
   const size_t cap = (size_t)run_capacity(n) * sizeof(RowRun);
   const size_t o_found = align256((size_t)n), o_runs = align256(o_found + cap);
-  const size_t o_del = align256(o_runs + cap);
+  const size_t o_slot = align256(o_runs + cap), o_list = align256(o_slot + (size_t)n * 4);
+  const size_t o_del = align256(o_list + (size_t)n * 4);
   const size_t bytes = o_del + (table ? 0 : (size_t)kMaxLag * std::max(B.nrows, 1) * sizeof(int2));
   int st = scratch_alloc(reinterpret_cast<void **>(&run_block), bytes, s);
   if (st) return st;
   member = reinterpret_cast<unsigned char *>(run_block);
   found = reinterpret_cast<RowRun *>(run_block + o_found);
   runs = reinterpret_cast<RowRun *>(run_block + o_runs);
+  bunch_slot = reinterpret_cast<int *>(run_block + o_slot);
+  bunch_list = reinterpret_cast<int *>(run_block + o_list);
   if (!table) t64.one.bdel = t32.one.bdel = reinterpret_cast<int2 *>(run_block + o_del);
   return NSPB_OK;
 }
@@ -318,14 +335,41 @@ int Call::alloc_runs() {
 int Call::build_programs() {
   for (int c = 0; c < 2; ++c) nruns[c] = run_block ? h.run.nruns[c] : 0;
   use_runs = nruns[0] + nruns[1] > 0;
+  nprog = nbunch = 0;
   if (!use_runs) return NSPB_OK;
-  int st = scratch_alloc(&progs, (size_t)h.run.nprog * run_prog_bytes(), s);
-  if (st) return st;
-  const cudaError_t e = launch_run_progs(structure_of(t64), found, rtab, h.run.nprog,
-                                         fp32_inputs(opts.precision), progs, &ctr->err, s);
+  nprog = h.run.nprog;
+  // the rows left over, where the runs took most of the row-group rows
+  long long taken = 0, left = 0;
+  for (int b = 0; b < kSymGroupBins; ++b) {
+    taken += h.sym_sub[b];
+    left += h.sym_counts[b] - h.sym_sub[b];
+  }
+  int st;
+  cudaError_t e;
+  if (left > 0 && taken >= left) {
+    e = launch_bunch_find(structure_of(t64), member, n, lim, row_nz, rtab, bunch_slot, bunch_list,
+                          ctr->sym_sub, s);
+    if (e != cudaSuccess) return cuda_fail(e);
+    launches += 3;
+    if ((st = fetch_counters())) return st;
+    nbunch = h.run.nbunch;
+  }
+  if ((st = scratch_alloc(&progs, (size_t)(nprog + nbunch) * run_prog_bytes(), s))) return st;
+  e = launch_run_progs(structure_of(t64), found, rtab, nprog, nbunch, fp32_inputs(opts.precision),
+                       progs, &ctr->err, s);
   if (e != cudaSuccess) return cuda_fail(e);
   ++launches;
   return NSPB_OK;
+}
+
+// The rows of runs and bunches get their counts (nz) and leave the numeric bins.
+cudaError_t Call::count_runs(int *nz, const int *crpt) {
+  cudaError_t e = launch_run_counts(found, h.run.nfound, runs, (int)run_capacity(n), rtab, progs, nz,
+                                    crpt, lim, ctr->num_sub, s);
+  if (e == cudaSuccess)
+    e = launch_bunch_counts(rtab, nprog, nbunch, bunch_list, progs, nz, crpt, lim, ctr->num_sub, s);
+  launches += 1 + (nbunch > 0);
+  return e;
 }
 
 void Call::drop_runs() {
@@ -336,6 +380,7 @@ void Call::drop_runs() {
   t64.one.bdel = t32.one.bdel = nullptr;
   use_runs = false;
   nruns[0] = nruns[1] = 0;
+  nprog = nbunch = 0;
 }
 
 // same: B is A, whose order the row walk of k_rowinfo checks.
@@ -377,7 +422,7 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
                           &ctr->long_rows, scan, s)) != cudaSuccess)
     return cuda_fail(e);
   if (run_block) {
-    if ((e = launch_run_find(structure_of(t64), member, n, lim, row_nz, found, runs, rtab,
+    if ((e = launch_run_find(structure_of(t64), member, n, lim, row_nz, found, rtab,
                              ctr->sym_sub, s)) != cudaSuccess)
       return cuda_fail(e);
     launches += 2;
@@ -408,7 +453,7 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
   long long map_bin_off[kSymGroupBins] = {};
   int map_stride[kSymGroupBins] = {};
   use_map = false;
-  if (map_wanted()) {
+  if (binned > 0 && map_wanted()) {
     long long total = 0;
     for (int b = 0; b < kSymGroupBins; ++b) {
       // quads of the map take at most 4/3 of a byte per product, plus alignment
@@ -467,10 +512,7 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
     ++launches;
   }
   if (use_runs) {
-    if ((e = launch_run_counts(runs, nruns, (int)run_capacity(n), rtab, progs, row_nz, nullptr, lim,
-                               ctr->num_sub, s)) != cudaSuccess)
-      return cuda_fail(e);
-    ++launches;
+    if ((e = count_runs(row_nz, nullptr)) != cudaSuccess) return cuda_fail(e);
   }
   mark(3);
   if ((e = launch_scan(row_nz, n, crpt, &ctr->total_nnz, tile_state, &ctr->tile_ctr, lim,
@@ -527,6 +569,15 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
                                   &ctr->ticket[30], s);
     if (e != cudaSuccess) return cuda_fail(e);
     launches += (nruns[0] > 0) + (nruns[1] > 0);
+    if (nbunch > 0) {
+      e = comp ? launch_numeric_comp_bunch(t32, rtab, nprog, nbunch, bunch_list, progs, crpt, ccol,
+                                           cval, nmax, &ctr->redo_count, &ctr->max_comp_deg,
+                                           &ctr->err, &ctr->ticket[28], s)
+               : launch_numeric_bunch(t64, rtab, nprog, nbunch, bunch_list, progs, crpt, ccol, cval,
+                                      &ctr->err, &ctr->ticket[28], s);
+      if (e != cudaSuccess) return cuda_fail(e);
+      launches += 2;
+    }
   }
   for (int b = 0; b < kNumBins; ++b) {
     const int c = todo[b];
@@ -614,7 +665,7 @@ int Call::prepare_numeric(const int *crpt) {
     if ((e = launch_rowinfo(structure_of(t64), n, a_nnz, lim, row_nz, nullptr, ctr->sym_counts,
                             &ctr->total_ip, nullptr, perm, &ctr->long_rows, scan, s)) !=
             cudaSuccess ||
-        (e = launch_run_find(structure_of(t64), member, n, lim, row_nz, found, runs, rtab,
+        (e = launch_run_find(structure_of(t64), member, n, lim, row_nz, found, rtab,
                              ctr->sym_sub, s)) != cudaSuccess)
       return cuda_fail(e);
     launches += 3;
@@ -628,10 +679,7 @@ int Call::prepare_numeric(const int *crpt) {
   if ((st = build_programs()) == NSPB_ERR_ALLOC) drop_runs();
   else if (st) return st;
   if (use_runs) {
-    if ((e = launch_run_counts(runs, nruns, (int)run_capacity(n), rtab, progs, nullptr, crpt, lim,
-                               ctr->num_sub, s)) != cudaSuccess)
-      return cuda_fail(e);
-    ++launches;
+    if ((e = count_runs(nullptr, crpt)) != cudaSuccess) return cuda_fail(e);
     if ((st = fetch_counters())) return st;
     for (int b = 0; b < 16; ++b) run_rows[b] = h.num_sub[b];
   }

@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstddef>
+
 #include "internal.h"
 
 namespace nspb {
@@ -27,7 +29,9 @@ struct DevCounters {
   int long_rows;     // rows listed for the block-per-row intermediate-product count
   int pad;
   int ticket[32];    // row tickets of the block-per-row launches (symbolic
-                     // bin b at b, numeric bin b at 16 + b; the runs at 30, 31)
+                     // bin b at b, numeric bin b at 16 + b; the runs at 30,
+                     // 31, the bunches at 28, 29)
+  // from here on only with row runs (Call::counter_bytes)
   int lag_count[4];  // B rows with a column shift at lag 1, 2, 3
   int sym_sub[16];   // rows of each symbolic bin that belong to a run
   int num_sub[16];   // rows of each numeric bin that do
@@ -100,13 +104,22 @@ struct Call {
   RowRun *found = nullptr, *runs = nullptr;
   RunTable rtab;
   void *progs = nullptr;       // pool block: one program a pattern
-  int run_rows[16] = {};       // rows of each numeric bin that belong to runs
+  int nprog = 0, nbunch = 0;   // patterns of the runs; bunches of other rows
+  int *bunch_slot = nullptr, *bunch_list = nullptr;
+  int run_rows[16] = {};       // rows of each numeric bin that belong to runs or bunches
   int64_t b_nnz = 0;           // entries of B over all products
+  // without runs the counters and the scratch are as large as they were before
+  // there were any: nspb_spgemm_noalloc serves as many rows
+  size_t counter_bytes() const {
+    return allow_runs ? sizeof(DevCounters) : offsetof(DevCounters, lag_count);
+  }
   bool runs_wanted() const;
   int alloc_runs();
   void drop_runs();
-  // After the counters are read: the programs of the patterns found.
+  // After the counters are read: the bunches (the counters are read again)
+  // and the programs of all patterns.
   int build_programs();
+  cudaError_t count_runs(int *nz, const int *crpt);
   // B's row order and, with runs, its column shifts
   cudaError_t check_b(bool same);
   // opts.timing: events around rowinfo, symbolic, scan, numeric

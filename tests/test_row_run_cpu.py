@@ -15,7 +15,7 @@ from nsp_b200.csr import HostCSR
 NO, ANY = None, "any"
 MAX_LAG, MAX_LEN, MAX_A, MAX_IP, RUN_MIN, BLOCK = 3, 128, 128, 1536, 6, 512
 SMALL_IP, REACH = 256, 512
-CLASS = {False: (50 * 1024, 8), True: (108 * 1024, 16)}  # shared memory, warps
+CLASS = {False: (50 * 1024, 8), True: (110000, 16)}  # shared memory, warps
 
 
 def shifts(B):
