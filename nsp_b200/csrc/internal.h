@@ -183,6 +183,7 @@ struct CompArgs {
                    // fp32 pairs; longer rows accumulate in fp64
   int *redo;       // counter of rows accumulated in fp64
   int *max_deg;    // largest A-row degree among the pair-accumulated rows
+  bool owned = false;  // k_num_flat: B rows hold no repeated column (else fp64 rows only)
 };
 
 // ---- rowinfo.cu -----------------------------------------------------------------
@@ -268,11 +269,13 @@ cudaError_t launch_symbolic_map(int bin, int lanes, const ProdTable<void> &t, co
 // tshift: the row-group bins use tables 2^tshift times their default size.
 // b_sorted: B rows strictly increasing (long rows take their column span
 // from the ends of the B rows they touch).
+// dcount: where given, the number of rows is read from the device (count is
+// an upper bound); bins below kNumLong only.
 cudaError_t launch_numeric_bin(int bin, int lanes, bool owned, bool b_sorted,
                                const ProdTable<double> &t, const ProdInfo &info,
                                const int *crpt, int *ccol, double *cval,
                                const int *rows, int count, int *err, int *ticket,
-                               int tshift, cudaStream_t s);
+                               int tshift, const int *dcount, cudaStream_t s);
 
 // Compensated numeric step (fp32 inputs): rows with at most nmax A entries
 // accumulate error-free fp32 pairs (TwoProduct + TwoSum) collapsed to fp64;
@@ -283,7 +286,20 @@ cudaError_t launch_numeric_comp_bin(int bin, int lanes, bool owned, bool b_sorte
                                     const ProdTable<float> &t, const ProdInfo &info,
                                     const int *crpt, int *ccol, double *cval, const int *rows,
                                     int count, int nmax, int *redo, int *max_deg, int *err,
-                                    int *ticket, int tshift, cudaStream_t s);
+                                    int *ticket, int tshift, const int *dcount, cudaStream_t s);
+
+// ---- numflat.cu -----------------------------------------------------------------
+// Numeric bin (bin < kNumLong) by sorting each row's products: for rows most
+// of whose products are entries of C of their own. Rows with more products
+// than the bin's kernel holds (about 1.25 times the bin's row limit) are
+// appended to over[*n_over] instead; B rows in any order.
+cudaError_t launch_numeric_flat(int bin, const ProdTable<double> &t, const int *crpt, int *ccol,
+                                double *cval, const int *rows, int count, int *over, int *n_over,
+                                int *err, cudaStream_t s);
+cudaError_t launch_numeric_comp_flat(int bin, bool owned, const ProdTable<float> &t,
+                                     const int *crpt, int *ccol, double *cval, const int *rows,
+                                     int count, int nmax, int *redo, int *max_deg, int *over,
+                                     int *n_over, int *err, cudaStream_t s);
 
 // ---- rowgroup.cu ----------------------------------------------------------------
 // Staged-walk numeric kernels of the row-group bins (numeric bins <

@@ -68,8 +68,9 @@ template <int G, int LOG2T, bool OWNED, typename VT, bool COMP, bool MULTI>
 __global__ void __launch_bounds__(256)
     k_num_group(const ProdTable<VT> src, const int *__restrict__ crpt, int *__restrict__ ccol,
                 double *__restrict__ cval, const int *__restrict__ rows, int count,
-                int *__restrict__ err, CompArgs comp) {
+                int *__restrict__ err, CompArgs comp, const int *__restrict__ dcount) {
   using C = NumGroupCfg<G, LOG2T>;
+  if (dcount) count = *dcount;
   extern __shared__ __align__(16) unsigned char smem_num[];
   auto tile = cg::tiled_partition<G>(cg::this_thread_block());
   const int g = threadIdx.x / G;
@@ -284,8 +285,10 @@ template <int LOG2T, typename VT, bool MULTI>
 __global__ void __launch_bounds__(kNumBlockThreads, num_block_minb(LOG2T))
     k_num_block(const ProdTable<VT> src, const int *__restrict__ crpt, int *__restrict__ ccol,
                 double *__restrict__ cval, const int *__restrict__ rows, int count,
-                int *__restrict__ err, int *__restrict__ redo, int *__restrict__ ticket) {
+                int *__restrict__ err, int *__restrict__ redo, int *__restrict__ ticket,
+                const int *__restrict__ dcount) {
   constexpr int T = 1 << LOG2T, H = T / 2, NB = T / 2;
+  if (dcount) count = *dcount;
   constexpr int PER = NB / kNumBlockThreads;
   extern __shared__ __align__(16) unsigned char smem_num[];
   double *vals = reinterpret_cast<double *>(smem_num);
@@ -609,22 +612,22 @@ static cudaError_t run_num_rank(const ProdTable<VT> &t, const ProdInfo &info, bo
 template <int G, int LOG2T, bool OWNED, typename VT, bool COMP>
 static cudaError_t run_num_group(const ProdTable<VT> &t, const int *crpt, int *ccol,
                                  double *cval, const int *rows, int count, int *err,
-                                 CompArgs comp, cudaStream_t s) {
+                                 CompArgs comp, const int *dcount, cudaStream_t s) {
   using C = NumGroupCfg<G, LOG2T>;
   auto kern = t.prod_of_row ? k_num_group<G, LOG2T, OWNED, VT, COMP, true>
                             : k_num_group<G, LOG2T, OWNED, VT, COMP, false>;
   const int grid = persistent_grid((const void *)kern, C::THREADS, C::SMEM, count, C::GPC);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
-  kern<<<grid, C::THREADS, C::SMEM, s>>>(t, crpt, ccol, cval, rows, count, err, comp);
+  kern<<<grid, C::THREADS, C::SMEM, s>>>(t, crpt, ccol, cval, rows, count, err, comp, dcount);
   return cudaGetLastError();
 }
 
 template <int G, bool OWNED, typename VT, bool COMP>
 static cudaError_t num_group_bin(int bin, const ProdTable<VT> &t, const int *crpt, int *ccol,
                                  double *cval, const int *rows, int count, int *err,
-                                 CompArgs comp, int tshift, cudaStream_t s) {
+                                 CompArgs comp, int tshift, const int *dcount, cudaStream_t s) {
 #define NSPB_NG(L2T) \
-  run_num_group<G, L2T, OWNED, VT, COMP>(t, crpt, ccol, cval, rows, count, err, comp, s)
+  run_num_group<G, L2T, OWNED, VT, COMP>(t, crpt, ccol, cval, rows, count, err, comp, dcount, s)
   // bin b holds rows of at most 16 << b entries; its table has 32 << (b + tshift)
   // slots (load <= 1/2 or 1/4), 1024 at most
   switch (std::min(5 + bin + tshift, 10)) {
@@ -641,13 +644,14 @@ static cudaError_t num_group_bin(int bin, const ProdTable<VT> &t, const int *crp
 template <int LOG2T, typename VT>
 static cudaError_t run_num_block(const ProdTable<VT> &t, const int *crpt, int *ccol,
                                  double *cval, const int *rows, int count, int *err, int *redo,
-                                 int *ticket, cudaStream_t s) {
+                                 int *ticket, const int *dcount, cudaStream_t s) {
   constexpr int T = 1 << LOG2T;
   const int smem = T * 12 + (T / 2) * 12 + (T / 2) * 4;
   auto kern = t.prod_of_row ? k_num_block<LOG2T, VT, true> : k_num_block<LOG2T, VT, false>;
   const int grid = persistent_grid((const void *)kern, kNumBlockThreads, smem, count, 1);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
-  kern<<<grid, kNumBlockThreads, smem, s>>>(t, crpt, ccol, cval, rows, count, err, redo, ticket);
+  kern<<<grid, kNumBlockThreads, smem, s>>>(t, crpt, ccol, cval, rows, count, err, redo, ticket,
+                                             dcount);
   return cudaGetLastError();
 }
 
@@ -655,10 +659,12 @@ template <typename VT, bool COMP>
 static cudaError_t numeric_bin_t(int bin, int lanes, bool owned, bool b_sorted,
                                  const ProdTable<VT> &t, const ProdInfo &info, const int *crpt,
                                  int *ccol, double *cval, const int *rows, int count, int *err,
-                                 CompArgs comp, int *ticket, int tshift, cudaStream_t s) {
+                                 CompArgs comp, int *ticket, int tshift, const int *dcount,
+                                 cudaStream_t s) {
   if (bin < kNumGroupBins) {
 #define NSPB_GB(GL, OW) \
-  num_group_bin<GL, OW, VT, COMP>(bin, t, crpt, ccol, cval, rows, count, err, comp, tshift, s)
+  num_group_bin<GL, OW, VT, COMP>(bin, t, crpt, ccol, cval, rows, count, err, comp, tshift, \
+                                  dcount, s)
     if (owned) {
       if (lanes == 8) return NSPB_GB(8, true);
       if (lanes == 16) return NSPB_GB(16, true);
@@ -675,33 +681,37 @@ static cudaError_t numeric_bin_t(int bin, int lanes, bool owned, bool b_sorted,
                             ticket, s);
   switch (bin) {
     case kNumGroupBins:
-      return run_num_block<11, VT>(t, crpt, ccol, cval, rows, count, err, redo, ticket, s);
+      return run_num_block<11, VT>(t, crpt, ccol, cval, rows, count, err, redo, ticket, dcount,
+                                   s);
     case kNumGroupBins + 1:
-      return run_num_block<12, VT>(t, crpt, ccol, cval, rows, count, err, redo, ticket, s);
+      return run_num_block<12, VT>(t, crpt, ccol, cval, rows, count, err, redo, ticket, dcount,
+                                   s);
     default:
-      return run_num_block<13, VT>(t, crpt, ccol, cval, rows, count, err, redo, ticket, s);
+      return run_num_block<13, VT>(t, crpt, ccol, cval, rows, count, err, redo, ticket, dcount,
+                                   s);
   }
 }
 
 cudaError_t launch_numeric_bin(int bin, int lanes, bool owned, bool b_sorted,
                                const ProdTable<double> &t, const ProdInfo &info,
                                const int *crpt, int *ccol, double *cval, const int *rows,
-                               int count, int *err, int *ticket, int tshift, cudaStream_t s) {
+                               int count, int *err, int *ticket, int tshift, const int *dcount,
+                               cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   return numeric_bin_t<double, false>(bin, lanes, owned, b_sorted, t, info, crpt, ccol, cval,
                                       rows, count, err, CompArgs{0, nullptr, nullptr}, ticket,
-                                      tshift, s);
+                                      tshift, dcount, s);
 }
 
 cudaError_t launch_numeric_comp_bin(int bin, int lanes, bool owned, bool b_sorted,
                                     const ProdTable<float> &t, const ProdInfo &info,
                                     const int *crpt, int *ccol, double *cval, const int *rows,
                                     int count, int nmax, int *redo, int *max_deg, int *err,
-                                    int *ticket, int tshift, cudaStream_t s) {
+                                    int *ticket, int tshift, const int *dcount, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   return numeric_bin_t<float, true>(bin, lanes, owned, b_sorted, t, info, crpt, ccol, cval, rows,
                                     count, err, CompArgs{nmax, redo, max_deg}, ticket, tshift,
-                                    s);
+                                    dcount, s);
 }
 
 }  // namespace nspb

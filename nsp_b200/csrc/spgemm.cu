@@ -552,7 +552,8 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
                          s)) != cudaSuccess)
       return cuda_fail(e);
     ++launches;
-    if ((e = order_block_bins(crpt, 1, todo, kNumGroupBins, kNumBins, off)) != cudaSuccess)
+    if ((e = order_block_bins(crpt, 1, todo, use_flat() ? kNumLong : kNumGroupBins, kNumBins,
+                              off)) != cudaSuccess)
       return cuda_fail(e);
   }
   // fp32 inputs: rows of at most nmax A entries accumulate in fp32 pairs, the
@@ -560,6 +561,14 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
   const bool comp = fp32_inputs(opts.precision);
   const int nmax = opts.precision == NSPB_PREC_FP32_COMP ? comp_nmax(opts.comp_tol) : 0;
   const bool staged = use_staged();
+  auto hash_bin = [&](int b, int g, const int *rows, int c, int *ticket, int tshift,
+                      const int *dcount) {
+    return comp ? launch_numeric_comp_bin(b, g, b_sorted, b_sorted, t32, info, crpt, ccol, cval,
+                                          rows, c, nmax, &ctr->redo_count, &ctr->max_comp_deg,
+                                          &ctr->err, ticket, tshift, dcount, s)
+                : launch_numeric_bin(b, g, b_sorted, b_sorted, t64, info, crpt, ccol, cval, rows,
+                                     c, &ctr->err, ticket, tshift, dcount, s);
+  };
   if (use_runs) {
     const int cap = (int)run_capacity(n);
     e = comp ? launch_numeric_comp_run(t32, runs, nruns, cap, progs, crpt, ccol, cval, nmax,
@@ -579,6 +588,12 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
       launches += 2;
     }
   }
+  // rows that the flat kernels leave, of the row-group bins and of the others
+  // (row_nz is free by now), and how many
+  const bool flat = use_flat();
+  int *over[2] = {row_nz, row_nz + off.v[kNumGroupBins]};
+  int *n_over[2] = {&ctr->ticket[26], &ctr->ticket[27]};
+  int flat_rows[2] = {0, 0};
   for (int b = 0; b < kNumBins; ++b) {
     const int c = todo[b];
     if (c <= 0) continue;
@@ -611,14 +626,28 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
       ++launches;
       continue;
     }
-    e = comp ? launch_numeric_comp_bin(b, lanes, b_sorted, b_sorted, t32, info, crpt, ccol, cval,
-                                       rows,
-                                       c, nmax, &ctr->redo_count, &ctr->max_comp_deg, &ctr->err,
-                                       ticket, tshift, s)
-             : launch_numeric_bin(b, lanes, b_sorted, b_sorted, t64, info, crpt, ccol, cval,
-                                  rows, c,
-                                  &ctr->err, ticket, tshift, s);
-    if (e != cudaSuccess) return cuda_fail(e);
+    if (b < kNumLong && flat) {
+      const int k = b >= kNumGroupBins;
+      e = comp ? launch_numeric_comp_flat(b, b_sorted, t32, crpt, ccol, cval, rows, c, nmax,
+                                          &ctr->redo_count, &ctr->max_comp_deg, over[k], n_over[k],
+                                          &ctr->err, s)
+               : launch_numeric_flat(b, t64, crpt, ccol, cval, rows, c, over[k], n_over[k],
+                                     &ctr->err, s);
+      if (e != cudaSuccess) return cuda_fail(e);
+      ++launches;
+      flat_rows[k] += c;
+      continue;
+    }
+    if ((e = hash_bin(b, lanes, rows, c, ticket, tshift, nullptr)) != cudaSuccess)
+      return cuda_fail(e);
+    ++launches;
+  }
+  for (int k = 0; k < 2; ++k) {
+    if (flat_rows[k] == 0) continue;
+    const int b = k ? kNumLong - 1 : kNumGroupBins - 1;
+    if ((e = hash_bin(b, 32, over[k], flat_rows[k], &ctr->ticket[16 + b], 0, n_over[k])) !=
+        cudaSuccess)
+      return cuda_fail(e);
     ++launches;
   }
   mark(6);

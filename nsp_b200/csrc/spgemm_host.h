@@ -30,7 +30,8 @@ struct DevCounters {
   int pad;
   int ticket[32];    // row tickets of the block-per-row launches (symbolic
                      // bin b at b, numeric bin b at 16 + b; the runs at 30,
-                     // 31, the bunches at 28, 29)
+                     // 31, the bunches at 28, 29; at 26, 27 the rows that
+                     // k_num_flat left to the hash kernels)
   // from here on only with row runs (Call::counter_bytes)
   int lag_count[4];  // B rows with a column shift at lag 1, 2, 3
   int sym_sub[16];   // rows of each symbolic bin that belong to a run
@@ -152,6 +153,14 @@ struct Call {
     if (opts.row_kernel & kNoRowTemplates) return 1;
     const int r = (opts.row_kernel >> 20) & 0xff;
     return r ? -r : kTemplateRun;
+  }
+  // Numeric bins up to kNumLong by sorting the products (numflat.cu): the rest
+  // of the automatic choice, rows whose products are mostly entries of C of
+  // their own. Their lists hold a quarter more products than entries; rows with
+  // more go to the hash kernels afterwards. Not in a two-call numeric step,
+  // which does not know the products (intprod 0).
+  bool use_flat() const {
+    return family() == 0 && opts.num_table_shift == 0 && intprod > 0 && !use_staged();
   }
   int rg_depth() const {
     const int d = (opts.row_kernel >> 8) & 0xff;
