@@ -264,6 +264,11 @@ cudaError_t launch_symbolic_map(int bin, int lanes, const ProdTable<void> &t, co
                                 int count, int *row_nz, int *err, const MapArgs &m,
                                 cudaStream_t s);
 
+// ---- symflat.cu -----------------------------------------------------------------
+// Symbolic bin < kSymGroupBins from flat product lists; B rows in any order.
+cudaError_t launch_symbolic_flat(int bin, const ProdTable<void> &t, const int *rows, int count,
+                                 int *row_nz, int *err, cudaStream_t s);
+
 // ---- numeric.cu -----------------------------------------------------------------
 // owned: B rows hold no duplicate columns (deterministic plain accumulation).
 // tshift: the row-group bins use tables 2^tshift times their default size.

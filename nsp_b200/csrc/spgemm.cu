@@ -197,6 +197,7 @@ void Call::set_table(const ProdTable<double> &d, const ProdTable<float> &f, cons
 }
 
 size_t Call::scratch_bytes() {
+  allow_runs = runs_wanted();  // no tables, and fewer counters to clear and read, without
   const size_t nn = (size_t)std::max(n, 1);
   off_row_nz = 0;
   off_perm = align256(off_row_nz + (nn + 1) * 4);
@@ -301,18 +302,20 @@ static BinOffsets offsets_of(const int *counts, int nb, int *nonempty, int *tota
 // to the library and A's rows are short enough on average for runs to hold
 // most of them. The search and the programs cost a chain of ten small launches,
 // so small products do without, unless row_kernel is 8: those of fewer than
-// about 24 million intermediate products (A's entries times B's mean row), or 6
+// about 24 million intermediate products (A's entries times B's mean row), or 8
 // million where B's rows are so short that the row-group kernels leave most
-// lanes idle. Measured, runs against none: 27-point 32^3 (21 M) 289 vs 321 us,
-// 24^3 (8.5 M) 282 vs 222, R (A P) of 60^3 (11 M) 396 vs 357; 7-point 64 x 50 x 50
-// (7.6 M) 244 vs 284, 32^3 (1.5 M) 214 vs 167, A P of 40^3 (7.4 M) 303 vs 332.
+// lanes idle. Measured, runs against none: 27-point 40^3 (42 M) 379 vs 497 us,
+// 30^3 (17 M) 297 vs 333, 24^3 (8.5 M) 280 vs 244, R (A P) of 80^3 (28 M) 507
+// vs 519, of 60^3 (11 M) 404 vs 262; B's rows of 4.5 and 7: A P of 48^3 (12 M)
+// 341 vs 390, of 40^3 (7.4 M) 310 vs 284, 7-point 64^3 (12.5 M) 286 vs 406,
+// 64 x 50 x 50 (7.6 M) 249 vs 314, 32^3 (1.5 M) 222 vs 170.
 bool Call::runs_wanted() const {
   if (!allow_runs || family() != 0 || (opts.row_kernel & kNoRowTemplates)) return false;
   if (n < 2 * kRunMin || a_nnz > (int64_t)kRunMaxA * n || (table && !info.bdel)) return false;
   if ((opts.row_kernel & 0xff) == 8) return true;
   if (info.brows <= 0) return false;
   const double mean = (double)b_nnz / (double)info.brows;
-  return (double)a_nnz * mean >= (mean < 8.0 ? 6e6 : 24e6);
+  return (double)a_nnz * mean >= (mean < 8.0 ? 8e6 : 24e6);
 }
 
 int Call::alloc_runs() {
@@ -490,6 +493,8 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
     if ((e = order_block_bins(row_nz, 0, todo, kSymGroupBins, kSymBins, off)) != cudaSuccess)
       return cuda_fail(e);
   }
+  // flat product lists unless the B rows fill the lanes of a row group
+  const bool flat = family() == 0 && (double)intprod < 0.75 * (double)lanes * (double)a_nnz;
   for (int b = 0; b < kSymBins; ++b) {
     const int c = todo[b];
     if (c <= 0) continue;
@@ -504,6 +509,8 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
       m.chunk = template_run();
       m.bshift = bshift;
       e = launch_symbolic_map(b, lanes, structure_of(t64), rows, c, row_nz, &ctr->err, m, s);
+    } else if (b < kSymGroupBins && flat) {
+      e = launch_symbolic_flat(b, structure_of(t64), rows, c, row_nz, &ctr->err, s);
     } else {
       e = launch_symbolic_bin(b, lanes, b_sorted, structure_of(t64), info, rows, c, row_nz,
                               &ctr->err, &ctr->ticket[b], s);

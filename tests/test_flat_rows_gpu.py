@@ -1,5 +1,5 @@
-"""Rows whose products are sorted as one list (k_num_flat): products of few
-repeated columns. Sums are formed in A-row order from zero, like the oracle's,
+"""Rows whose products are one flat list: counted (k_sym_flat, row_products) and,
+where few columns repeat, sorted (k_num_flat). Sums are formed in A-row order from zero, like the oracle's,
 so values are compared bit for bit. Sizes: row lengths at the edges of the
 bins and of the lists, empty rows of A and B, B rows longer than a block,
 repeated columns inside a bucket and at the ends of a row, rows whose columns
@@ -65,26 +65,56 @@ def clusters(rng):
     return A, B
 
 
+def counts(rng):
+    """Products at the edges of the symbolic bins; rows with many more products than C has columns."""
+    lens = [d for e in (24, 48, 96, 192, 384, 768, 1536, 3072, 6144) for d in (e - 1, e, e + 1)]
+    k, m = 7000, 40_009
+    A = from_rows([pick(rng, k, d) for d in lens], k, rng)
+    B = from_rows([c[None] for c in pick(rng, m, k)], m, rng)
+    return A, B
+
+
+def narrow(rng):
+    k, m = 500, 33
+    B = from_rows([pick(rng, m, rng.integers(0, 20)) for _ in range(k)], m, rng)
+    A = from_rows([pick(rng, k, d) for d in (0, 1, 2, 3, 4, 40, 100, 300, 500)], k, rng)
+    return A, B
+
+
+def heavy(rng):
+    """Rounds of over 16384 products, of 1024 entries and of one more, B rows of 1024 entries."""
+    k, m = 3000, 300_007
+    brows = [pick(rng, m, rng.integers(0, 60)) for _ in range(k - 4)]
+    brows += [pick(rng, m, d) for d in (1023, 1024, 1025, 5000)]
+    arows = [pick(rng, k - 4, d) for d in (300, 1023, 1024, 1025, 2500)]
+    arows += [np.append(pick(rng, k - 4, d), np.arange(k - 4, k)) for d in (0, 200, 1020, 1024)]
+    return from_rows(arows, k, rng), from_rows(brows, m, rng)
+
+
 def as32(h):
     return HostCSR(h.nrows, h.ncols, h.rowptr, h.col, h.val.astype(np.float32))
 
 
 def check(A, B, precision, exact=True):
     X, Y = (A, B) if precision == "fp64" else (as32(A), as32(B))
-    C = nb.spgemm(X.to_device(), Y.to_device(), precision=precision).to_host()
+    dA, dB = X.to_device(), Y.to_device()
+    C = nb.spgemm(dA, dB, precision=precision).to_host()
+    rp2, nnz = nb.spgemm_symbolic(dA, dB)
+    C2 = nb.spgemm_numeric(dA, dB, rp2, nnz, precision=precision).to_host()
     rp, col, val = oracle.spgemm(A, B)
-    assert_same_structure(C.rowptr, C.col, rp, col)
     bound = oracle.absbound(A, B, rp, col)
     tol = {"fp64": 2.0**-50, "fp32w": 2.0**-50, "fp32c": 1e-10}[precision]
-    assert np.all(np.abs(C.val - val) <= tol * np.maximum(bound, 1e-300) * 40)
-    if exact and precision != "fp32c":
-        small = np.diff(rp) <= 512  # longer rows left to the hash kernels add in any order
-        keep = np.repeat(small, np.diff(rp))
-        assert_bitwise(C.val[keep], val[keep])
+    for c in (C, C2):
+        assert_same_structure(c.rowptr, c.col, rp, col)
+        assert np.all(np.abs(c.val - val) <= tol * np.maximum(bound, 1e-300) * 40)
+        # longer rows of many products of few columns take kernels that add in any order
+        if exact and precision != "fp32c":
+            keep = np.repeat(np.diff(rp) <= 512, np.diff(rp))
+            assert_bitwise(c.val[keep], val[keep])
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32w", "fp32c"])
-@pytest.mark.parametrize("make", [edges, mixed, clusters])
+@pytest.mark.parametrize("make", [edges, mixed, clusters, counts, narrow, heavy])
 def test_rows(cuda, make, precision):
     check(*make(np.random.default_rng(5)), precision)
 
