@@ -214,117 +214,144 @@ __device__ __forceinline__ double ldv_stream(const float *p) {
   return (double)v;
 }
 
-// Shared state of row_products: a queue of one round's A entries {B row
-// start, B row end, A value as two ints} and two sets of counters {medium
-// entries, long entries, medium cursor}, used in alternate rounds so that one
-// set is cleared while the other is in use. Counters start at zero.
+// Shared state of row_products: one round's A entries, those with B rows
+// shorter than the block from the front (place of the first product, distance
+// from a product's place to its B entry, A value), the others from the back
+// (start and end of the B row, A value); the front entry of the first of each
+// 32 products of a window; counters, zero at the start.
+constexpr int kRowWindow = 512;  // 32-product pieces per window
 template <int THREADS>
 struct RowQueue {
-  int4 q[THREADS];
-  int ctr[2][3];
+  double a[THREADS];
+  int start[THREADS], shift[THREADS];
+  unsigned red[32];
+  int big;
+  unsigned short first[kRowWindow];
 };
 
 template <int THREADS>
 __device__ __forceinline__ void row_queue_init(RowQueue<THREADS> &rq) {
-  if (threadIdx.x < 6) (&rq.ctr[0][0])[threadIdx.x] = 0;
+  if (threadIdx.x == 0) rq.big = 0;
 }
 
 // Every product of one A row, spread evenly over a block of THREADS threads
 // whatever the lengths of the B rows it touches (power-law matrices mix rows
 // of one entry with hub rows of 10^4 and more). The A row is taken in rounds
-// of THREADS entries, one per thread:
-//   - a B row of at most kRowSmall entries (4 when the round holds fewer than
-//     THREADS/4 entries) is walked by its thread, four entries' loads at a
-//     time: up to THREADS independent gather chains in flight;
-//   - a longer B row goes to a queue; warps take queued rows one at a time
-//     from a shared cursor, lanes over the row's entries;
-//   - a B row of THREADS entries or more is walked by the whole block, thread
-//     t taking the products whose index in the round's concatenation of such
-//     rows is t mod THREADS.
+// of THREADS entries. B rows of THREADS entries or more are walked by the
+// whole block, thread t taking the products whose index in the concatenation
+// of such rows is t mod THREADS. The products of all the others form one list
+// whose places a scan of their lengths gives; warps take pieces of 32
+// consecutive products, lane l the product l of the piece, so that every lane
+// works and neighbours read neighbouring B entries. U pieces' loads are in
+// flight at a time in each warp. ROWPROD_FIG
 // f(c, a, b) gets the B entry's column, the A value and the B value (values 0
 // when aval / bval are null). Every thread of the block must call this with
 // the same (a0, a1) after a block barrier, and a block barrier must separate
 // two calls.
-#ifndef NSPB_ROW_SMALL
-#define NSPB_ROW_SMALL 16
-#endif
-constexpr int kRowSmall = NSPB_ROW_SMALL;  // longest B row one thread walks alone
-
-template <int THREADS, typename VT, typename F>
+template <int THREADS, int U, typename VT, typename F>
 __device__ __forceinline__ void row_products(const int *__restrict__ acol,
                                              const VT *__restrict__ aval,
                                              const int *__restrict__ brpt,
                                              const int *__restrict__ bcol,
                                              const VT *__restrict__ bval, int a0, int a1,
                                              RowQueue<THREADS> &rq, F &&f) {
-  static_assert((THREADS & (THREADS - 1)) == 0, "THREADS must be a power of two");
-  const int lane = threadIdx.x & 31;
+  static_assert((THREADS & (THREADS - 1)) == 0 && THREADS <= 1024,
+                "a power of two; the packed scan holds 20 bits of products");
+  constexpr int NW = THREADS / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   auto bv = [&](int e) -> double { return bval ? ldv(bval + e) : 0.0; };
-  // entries [e, end) with stride S, two loads in flight per thread
-  auto strided = [&](int e, int end, double a, auto S) {
-    constexpr int kS = decltype(S)::value;
-    for (; e + kS < end; e += 2 * kS) {
-      const int c0 = __ldg(bcol + e), c1 = __ldg(bcol + e + kS);
-      const double b0 = bv(e), b1 = bv(e + kS);
+  // entries [e, end) with stride THREADS, two loads in flight per thread
+  auto strided = [&](int e, int end, double a) {
+    for (; e + THREADS < end; e += 2 * THREADS) {
+      const int c0 = __ldg(bcol + e), c1 = __ldg(bcol + e + THREADS);
+      const double b0 = bv(e), b1 = bv(e + THREADS);
       f(c0, a, b0);
       f(c1, a, b1);
     }
     if (e < end) f(__ldg(bcol + e), a, bv(e));
   };
-  int par = 0;
-  for (int jr = a0; jr < a1; jr += THREADS, par ^= 1) {  // uniform across the block
-    const int small_max = min(THREADS, a1 - jr) * 4 >= THREADS ? kRowSmall : 4;
+  for (int jr = a0; jr < a1; jr += THREADS) {  // uniform across the block
     const int j = jr + (int)threadIdx.x;
+    int len = 0, s0 = 0;
+    double a = 0.0;
     if (j < a1) {
       const int k = ld_stream(acol + j);
-      const double a = aval ? ldv_stream(aval + j) : 0.0;
-      const int s0 = __ldg(brpt + k), s1 = __ldg(brpt + k + 1);
-      if (s1 - s0 <= small_max) {
-        int e = s0;
-        for (; e + 4 <= s1; e += 4) {
-          const int c0 = __ldg(bcol + e), c1 = __ldg(bcol + e + 1);
-          const int c2 = __ldg(bcol + e + 2), c3 = __ldg(bcol + e + 3);
-          const double b0 = bv(e), b1 = bv(e + 1), b2 = bv(e + 2), b3 = bv(e + 3);
-          f(c0, a, b0);
-          f(c1, a, b1);
-          f(c2, a, b2);
-          f(c3, a, b3);
-        }
-        for (; e < s1; ++e) f(__ldg(bcol + e), a, bv(e));
-      } else {
-        const int big = (s1 - s0 >= THREADS) ? 1 : 0;
-        const int slot = atomicAdd(&rq.ctr[par][big], 1);
-        rq.q[big ? THREADS - 1 - slot : slot] =
-            make_int4(s0, s1, __double2loint(a), __double2hiint(a));
-      }
+      if (aval) a = ldv_stream(aval + j);
+      s0 = __ldg(brpt + k);
+      len = __ldg(brpt + k + 1) - s0;
     }
+    if (len >= THREADS) {
+      const int slot = THREADS - 1 - atomicAdd(&rq.big, 1);
+      rq.start[slot] = s0;
+      rq.shift[slot] = s0 + len;
+      rq.a[slot] = a;
+      len = 0;
+    }
+    // (entries before, products before) of this thread's entry
+    const unsigned v = len > 0 ? 1u << 20 | (unsigned)len : 0u;
+    unsigned incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    if (lane == 31) rq.red[warp] = incl;
     __syncthreads();
-    // the other counter set was last read before the previous round's closing
-    // barrier and is next written after this round's
-    if (threadIdx.x == 0) rq.ctr[par ^ 1][0] = rq.ctr[par ^ 1][1] = rq.ctr[par ^ 1][2] = 0;
-    const int nm = rq.ctr[par][0], nb = rq.ctr[par][1];
-    for (;;) {
-      int i = 0;
-      if (lane == 0) i = atomicAdd(&rq.ctr[par][2], 1);
-      i = __shfl_sync(0xffffffffu, i, 0);
-      if (i >= nm) break;
-      const int4 v = rq.q[i];
-      strided(v.x + lane, v.y, __hiloint2double(v.w, v.z), std::integral_constant<int, 32>());
+    const unsigned mine = lane < NW ? rq.red[lane] : 0u;
+    const unsigned all = __reduce_add_sync(0xffffffffu, mine);
+    const unsigned ex = incl - v + __reduce_add_sync(0xffffffffu, lane < warp ? mine : 0u);
+    const int total = (int)(all & 0xfffffu), ne = (int)(all >> 20);
+    const int p = (int)(ex & 0xfffffu), t = (int)(ex >> 20);
+    if (len > 0) {
+      rq.start[t] = p;
+      rq.shift[t] = s0 - p;
+      rq.a[t] = a;
     }
+    const int c_end = (p + len + 31) >> 5;  // pieces that start in this entry: [c_at, c_end)
+    int c_at = (p + 31) >> 5;
+    const int pieces = (total + 31) >> 5;
+    for (int w0 = 0; w0 < pieces; w0 += kRowWindow) {
+      const int wn = min(pieces - w0, kRowWindow);
+      for (; c_at < min(c_end, w0 + wn); ++c_at) rq.first[c_at - w0] = (unsigned short)t;
+      __syncthreads();
+      for (int c = warp; c < wn; c += NW * U) {
+        int e[U], col[U];
+        double av[U], b[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          e[u] = -1;
+          if (c + u * NW < wn) {
+            const int p0 = (w0 + c + u * NW) * 32, t0 = rq.first[c + u * NW];
+            const int st = t0 + 1 + lane < ne ? rq.start[t0 + 1 + lane] - p0 : 32;
+            const unsigned m = __reduce_or_sync(0xffffffffu, st < 32 ? 1u << st : 0u);
+            const int x = t0 + __popc(m & (0xffffffffu >> (31 - lane)));
+            if (p0 + lane < total) {
+              e[u] = p0 + lane + rq.shift[x];
+              col[u] = __ldg(bcol + e[u]);
+              b[u] = bv(e[u]);
+              av[u] = aval ? rq.a[x] : 0.0;
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (e[u] >= 0) f(col[u], av[u], b[u]);
+      }
+      if (w0 + kRowWindow < pieces) __syncthreads();  // first[]
+    }
+    const int nb = rq.big;
     unsigned pos = 0;  // products of the long rows before row i, mod 2^32
     for (int i = 0; i < nb; ++i) {
-      const int4 v = rq.q[THREADS - 1 - i];
-      const int first = (int)((threadIdx.x - pos) & (unsigned)(THREADS - 1));
-      strided(v.x + first, v.y, __hiloint2double(v.w, v.z),
-              std::integral_constant<int, THREADS>());
-      pos += (unsigned)(v.y - v.x);
+      const int q = THREADS - 1 - i, b0 = rq.start[q], b1 = rq.shift[q];
+      const int skip = (int)((threadIdx.x - pos) & (unsigned)(THREADS - 1));
+      strided(b0 + skip, b1, rq.a[q]);
+      pos += (unsigned)(b1 - b0);
     }
     __syncthreads();
+    // read again after the next round's first barrier, or the caller's
+    if (threadIdx.x == 0) rq.big = 0;
+    if (jr + THREADS < a1) __syncthreads();
   }
-  // counters of the last round (the other set was cleared during it); the
-  // caller's barrier before the next call orders this
-  if (a1 > a0 && threadIdx.x == 0)
-    rq.ctr[par ^ 1][0] = rq.ctr[par ^ 1][1] = rq.ctr[par ^ 1][2] = 0;
 }
 
 // Intermediate products of one A row and the range of columns they can
@@ -486,7 +513,9 @@ __device__ __forceinline__ void with_cols(bool staged, int skew, const int *word
   else if (skew == 5) body(ColSkewed{words, e0});
   else body(ColFlat{words, e0});
 }
-// Rows of a tile so that most tiles of a matrix of this mean row fit.
+// Rows of a tile so that most tiles of a matrix of this mean row fit. (Smaller
+// tiles for small matrices, two blocks an SM, made k_rowinfo slower: 8.2 -> 10.4
+// us for a 7-point 32^3, 8.8 -> 14.2 for 33000 rows of 27.)
 inline int tile_rows(double mean) {
   int r = kTileThreads;
   while (r > 32 && r * mean > 0.9 * kTileCols) r >>= 1;

@@ -525,7 +525,7 @@ __global__ void __launch_bounds__(kWideThreads, MINB)
       for (int q = threadIdx.x; q < (1 << kWideLog2T); q += kWideThreads) table[q] = kEmpty;
       __syncthreads();
       int nz = 0;
-      row_products<kWideThreads>(acol, (const double *)nullptr, brpt, bcol,
+      row_products<kWideThreads, (MINB > 1 ? 2 : 4)>(acol, (const double *)nullptr, brpt, bcol,
                                  (const double *)nullptr, a0, a1, rq,
                                  [&](int c, double, double) {
                                    nz += sym_insert<kWideLog2T, true>(table, c, err);
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(kWideThreads, MINB)
         const int base = (int)w0;
         for (int q = threadIdx.x; q < words; q += kWideThreads) bm[q] = 0u;
         __syncthreads();
-        row_products<kWideThreads>(acol, (const double *)nullptr, brpt, bcol,
+        row_products<kWideThreads, (MINB > 1 ? 2 : 4)>(acol, (const double *)nullptr, brpt, bcol,
                                    (const double *)nullptr, a0, a1, rq,
                                    [&](int c, double, double) {
                                      const unsigned d = (unsigned)(c - base);
