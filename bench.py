@@ -37,10 +37,10 @@ sys.path.insert(0, ROOT)
 
 L = 128
 SEED = 20261203
-# the row-group kernels the default call runs (dominant launches of the stencil
-# product): from entry maps when the call recorded them, else the staged walk
-NUM_KERNEL = {True: "k_num_map", False: "k_num_rg"}
-SYM_KERNEL = {True: "k_sym_map", False: "k_sym_group"}
+# the kernels the default call runs (dominant launches of the stencil product):
+# from entry maps when the call recorded them (small grids), else row runs
+NUM_KERNEL = {True: "k_num_map", False: "k_num_run"}
+SYM_KERNEL = {True: "k_sym_map", False: "k_run_key"}
 METRIC = "SpGEMM GFLOP/s, C=A*A, 27-point stencil 128^3, fp64"
 WORKLOAD = "stencil27_128^3_AxA_fp64"
 
