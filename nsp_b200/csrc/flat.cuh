@@ -59,18 +59,15 @@ __device__ __forceinline__ int flat_entries(const FlatTab &ft, const int *acol, 
   constexpr int TH = 32 * W;
   static_assert(TH <= 512, "the packed scan holds 10 bits of entries");
   int total = 0, ne = 0;
-  for (int base = a0;; base += TH) {
-    int len = 0, s0 = 0;
-    double av = 0.0;
-    if (base + tid < a1) {
-      const int k = ld_stream(acol + base + tid);
-      if (aval) av = ldv_stream(aval + base + tid);
-      s0 = __ldg(brpt + k);
-      len = min(__ldg(brpt + k + 1) - s0, cap + 1);
-    }
-    unsigned sum;
-    const unsigned ex = flat_scan<W>((unsigned)len | (len > 0 ? 1u << 22 : 0u), ft.red, warp, lane,
-                                     &sum);
+  // start and (clamped) length of the B row of entry base + tid, and its A value
+  auto load = [&](int base, int &s0, double &av) {
+    if (base + tid >= a1) return 0;
+    const int k = ld_stream(acol + base + tid);
+    if (aval) av = ldv_stream(aval + base + tid);
+    s0 = __ldg(brpt + k);
+    return min(__ldg(brpt + k + 1) - s0, cap + 1);
+  };
+  auto enter = [&](unsigned ex, int len, int s0, double av) {
     const int p = total + (int)(ex & 0x3fffffu), t = ne + (int)(ex >> 22);
     if (len > 0 && p + len <= cap) {
       ft.start[t] = p;
@@ -78,6 +75,33 @@ __device__ __forceinline__ int flat_entries(const FlatTab &ft, const int *acol, 
       if (aval) ft.a[t] = av;
       for (int c = (p + 31) >> 5; c << 5 < p + len; ++c) ft.first[c] = (unsigned short)t;
     }
+  };
+  // one warp has them all: the others wait for the sums instead of scanning
+  // zeros beside it (random 100003 x 80021 x 120011, the whole product: 878 -> 857 us)
+  if (W > 1 && a1 - a0 <= 32) {
+    if (warp == 0) {
+      int s0 = 0;
+      double av = 0.0;
+      const int len = load(a0, s0, av);
+      unsigned sum;
+      const unsigned ex = flat_scan<1>((unsigned)len | (len > 0 ? 1u << 22 : 0u), ft.red, 0, lane,
+                                       &sum);
+      enter(ex, len, s0, av);
+      if (lane == 0) ft.red[0] = sum;
+    }
+    __syncthreads();
+    const unsigned sum = ft.red[0];
+    *entries = (int)(sum >> 22);
+    return (int)(sum & 0x3fffffu);
+  }
+  for (int base = a0;; base += TH) {
+    int s0 = 0;
+    double av = 0.0;
+    const int len = load(base, s0, av);
+    unsigned sum;
+    const unsigned ex = flat_scan<W>((unsigned)len | (len > 0 ? 1u << 22 : 0u), ft.red, warp, lane,
+                                     &sum);
+    enter(ex, len, s0, av);
     total += (int)(sum & 0x3fffffu);
     ne += (int)(sum >> 22);
     if (total > cap || base + TH >= a1) break;

@@ -16,14 +16,14 @@
 //
 // Bound: instruction issue (64% of the slots) and shared-memory wavefronts
 // (60% of the data pipe), at 57% occupancy by registers; DRAM is at 10%. A
-// block a row keeps the rows' latencies apart; four warps for 257..512
-// entries, because with two and twice the products a thread the unrolled code
-// no longer fits the instruction cache (no-instruction stalls 7 of 16 cycles,
-// 417 us against 322 us with four). Measured on 100003 x 80021 x 120011 with
+// block a row keeps the rows' latencies apart; four warps and five products a
+// thread for 257..512 entries (259 us): with two warps and ten products the
+// unrolled code no longer fits the instruction cache (377 us), with eight warps
+// and three products every warp's work for the row as a whole weighs more (343). Measured on 100003 x 80021 x 120011 with
 // 4..32 entries a row (rows of 257..512 entries, 48800 of them): hash table,
 // compaction and bucket sort 694 us; products in wide buckets with a rank 322
-// us; bitmaps 259 us. All rows of that product 1160 -> 504 us; of 20 such
-// products of 1000..40000 rows in one call 4370 -> 2120 us.
+// us; bitmaps 259 us. All rows of that product 1160 -> 490 us; of 20 such
+// products of 1000..40000 rows in one call 4370 -> 2090 us.
 #include "flat.cuh"
 #include "internal.h"
 #include "launch_util.h"

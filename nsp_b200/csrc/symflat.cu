@@ -7,7 +7,8 @@
 // in flight at a time. Here all lanes have a product, and all products of a
 // thread are loaded before the first is inserted. Bound: issue and latency of
 // the inserts; the table has at least twice the products, so that most take
-// one exchange (reading the slot first made it slower: 121 -> 134 us below).
+// one exchange (reading the slot first made it slower: 121 -> 134 us below; so did twelve
+// products a thread with half the warps, 150, and three with twice the warps, 157).
 // Measured, row-group kernel -> this one: rows of 385..768 products of a random
 // product (4..32 entries a row) 163 -> 121 us, all rows of it 366 -> 250; 20
 // such products in one call 1151 -> 861; power-law 1M, rows of up to 3072
