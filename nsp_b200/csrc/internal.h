@@ -184,6 +184,7 @@ struct CompArgs {
   int *redo;       // counter of rows accumulated in fp64
   int *max_deg;    // largest A-row degree among the pair-accumulated rows
   bool owned = false;  // k_num_flat: B rows hold no repeated column (else fp64 rows only)
+  int most = 0x7fffffff;  // runs and bunches: entries of the longest row summed in pairs
 };
 
 // ---- rowinfo.cu -----------------------------------------------------------------
@@ -376,7 +377,7 @@ cudaError_t launch_numeric_bunch(const ProdTable<double> &t, const RunTable &rt,
                                  int *ccol, double *cval, int *err, int *ticket, cudaStream_t s);
 cudaError_t launch_numeric_comp_bunch(const ProdTable<float> &t, const RunTable &rt, int nprog,
                                       int nbunch, const int *list, const void *progs,
-                                      const int *crpt, int *ccol, double *cval, int nmax,
+                                      const int *crpt, int *ccol, double *cval, int nmax, int most,
                                       int *redo, int *max_deg, int *err, int *ticket,
                                       cudaStream_t s);
 // The runs by program (runs: small ones from the front, large ones from the
@@ -391,6 +392,7 @@ cudaError_t launch_numeric_run(const ProdTable<double> &t, const RowRun *runs,
                                int *ccol, double *cval, int *err, int *ticket, cudaStream_t s);
 cudaError_t launch_numeric_comp_run(const ProdTable<float> &t, const RowRun *runs,
                                     const int (&nruns)[2], int cap, const void *progs,
-                                    const int *crpt, int *ccol, double *cval, int nmax, int *redo,
-                                    int *max_deg, int *err, int *ticket, cudaStream_t s);
+                                    const int *crpt, int *ccol, double *cval, int nmax, int most,
+                                    int *redo, int *max_deg, int *err, int *ticket,
+                                    cudaStream_t s);
 }  // namespace nspb

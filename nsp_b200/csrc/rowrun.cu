@@ -1247,6 +1247,15 @@ __device__ __forceinline__ void run_walk(const uint2 *prog, int w0, int w1, cons
   }
 }
 
+// Compensated mode: whether rows of na A entries and n entries of C sum in fp32
+// pairs. The rows that the other kernels sum in pairs, so that a row's sums and
+// its bound do not depend on whether it is in a run: those of the row-group
+// bins (at most comp.most entries), over B rows without repeated columns
+// (comp.nmax is 0 otherwise), where an entry has at most na products.
+__device__ __forceinline__ bool run_pairs(const CompArgs &comp, int na, int n) {
+  return na <= comp.nmax && n <= comp.most;
+}
+
 // What the look-up warp leaves for a tile.
 struct RunTile {
   int prog;   // -1: no more tiles
@@ -1321,7 +1330,7 @@ __global__ void __launch_bounds__((RunCfg<CLASS>::WARPS + RunCfg<CLASS>::LOOK) *
       const int arow = run_arow(na, sizeof(VT)) / (int)sizeof(VT);
       const bool bulk_c = s == 1 && (n & 1) && (reinterpret_cast<size_t>(cval) & 15) == 0;
       if (COMP) {
-        if (na <= comp.nmax) max_deg = max(max_deg, na);
+        if (run_pairs(comp, na, n)) max_deg = max(max_deg, na);
         else redo += len;
       }
       for (int r0 = 0; r0 < len && !lost; r0 += L) {
@@ -1507,7 +1516,7 @@ __global__ void __launch_bounds__((RunCfg<CLASS>::WARPS + RunCfg<CLASS>::LOOK) *
       const int l = rg * 32 + lane;
       const int ll = min(l, cnt - 1);
       const bool write = l < cnt;
-      const bool pair = COMP && na <= comp.nmax;
+      const bool pair = COMP && run_pairs(comp, na, n);
       const char *al = reinterpret_cast<const char *>(sm.as + tile.ao[ll]);
       double *ol = out0 + (size_t)ll * npad;
       const char *bl = reinterpret_cast<const char *>(sm.bs + (pstep > 0 ? pstep : 0) * ll);
@@ -1594,10 +1603,11 @@ cudaError_t launch_numeric_run(const ProdTable<double> &t, const RowRun *runs,
 
 cudaError_t launch_numeric_comp_run(const ProdTable<float> &t, const RowRun *runs,
                                     const int (&nruns)[2], int cap, const void *progs,
-                                    const int *crpt, int *ccol, double *cval, int nmax, int *redo,
-                                    int *max_deg, int *err, int *ticket, cudaStream_t s) {
+                                    const int *crpt, int *ccol, double *cval, int nmax, int most,
+                                    int *redo, int *max_deg, int *err, int *ticket,
+                                    cudaStream_t s) {
   return run_num_runs<float, true>(t, runs, nruns, cap, progs, crpt, ccol, cval, err,
-                                   CompArgs{nmax, redo, max_deg}, ticket, s);
+                                   CompArgs{nmax, redo, max_deg, false, most}, ticket, s);
 }
 
 // ---- numeric phase of the bunches --------------------------------------------------
@@ -1649,7 +1659,7 @@ __global__ void __launch_bounds__(RunCfg<CLASS>::WARPS * 32, RunCfg<CLASS>::MINB
       for (int i = tid; i < P; i += THREADS) term[i] = pg.term[i];
       for (int i = tid; i <= na; i += THREADS) before[i] = pg.before[i];
     }
-    const bool pair = COMP && na <= comp.nmax;
+    const bool pair = COMP && run_pairs(comp, na, n);
     if (COMP && tid == 0) {
       if (pair) max_deg = max(max_deg, na);
       else redo += cnt;
@@ -1738,11 +1748,11 @@ cudaError_t launch_numeric_bunch(const ProdTable<double> &t, const RunTable &rt,
 
 cudaError_t launch_numeric_comp_bunch(const ProdTable<float> &t, const RunTable &rt, int nprog,
                                       int nbunch, const int *list, const void *progs,
-                                      const int *crpt, int *ccol, double *cval, int nmax,
+                                      const int *crpt, int *ccol, double *cval, int nmax, int most,
                                       int *redo, int *max_deg, int *err, int *ticket,
                                       cudaStream_t s) {
   if (nbunch <= 0) return cudaSuccess;
-  const CompArgs comp{nmax, redo, max_deg};
+  const CompArgs comp{nmax, redo, max_deg, false, most};
   cudaError_t e = run_num_bunch<1, float, true>(t, rt, nprog, nbunch, list, progs, crpt, ccol,
                                                 cval, err, comp, ticket + 1, s);
   if (e != cudaSuccess) return e;

@@ -578,8 +578,10 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
   };
   if (use_runs) {
     const int cap = (int)run_capacity(n);
-    e = comp ? launch_numeric_comp_run(t32, runs, nruns, cap, progs, crpt, ccol, cval, nmax,
-                                       &ctr->redo_count, &ctr->max_comp_deg, &ctr->err,
+    // pairs for the rows that the row-group kernels sum in pairs
+    const int pair_a = b_sorted ? nmax : 0, pair_c = lim.num[kNumGroupBins - 1];
+    e = comp ? launch_numeric_comp_run(t32, runs, nruns, cap, progs, crpt, ccol, cval, pair_a,
+                                       pair_c, &ctr->redo_count, &ctr->max_comp_deg, &ctr->err,
                                        &ctr->ticket[30], s)
              : launch_numeric_run(t64, runs, nruns, cap, progs, crpt, ccol, cval, &ctr->err,
                                   &ctr->ticket[30], s);
@@ -587,7 +589,7 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
     launches += (nruns[0] > 0) + (nruns[1] > 0);
     if (nbunch > 0) {
       e = comp ? launch_numeric_comp_bunch(t32, rtab, nprog, nbunch, bunch_list, progs, crpt, ccol,
-                                           cval, nmax, &ctr->redo_count, &ctr->max_comp_deg,
+                                           cval, pair_a, pair_c, &ctr->redo_count, &ctr->max_comp_deg,
                                            &ctr->err, &ctr->ticket[28], s)
                : launch_numeric_bunch(t64, rtab, nprog, nbunch, bunch_list, progs, crpt, ccol, cval,
                                       &ctr->err, &ctr->ticket[28], s);
