@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "../../include/nspb.h"
+#include "runrules.h"
 
 namespace nspb {
 
@@ -136,8 +137,7 @@ constexpr int kMaxLag = 3;
 constexpr int kNoShift = (int)0x80000000;
 constexpr int kAnyShift = 0x7fffffff;
 constexpr int kShiftMaxLen = 128;  // longer B rows are not compared
-constexpr int kRunMaxA = 128;      // A entries of a row in a run
-constexpr int kRunMaxIp = 1536;    // products of a row in a run
+// kRunMaxA, kRunMaxIp: runrules.h
 constexpr int kRunMin = 6;         // rows of the shortest run
 // A run: rows row0, row0 + s, ..., `len` of them; meta = s | sigma << 2 | len << 4.
 struct RowRun {

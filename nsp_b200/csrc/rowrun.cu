@@ -468,14 +468,14 @@ __global__ void __launch_bounds__(256)
         if (t < na) {
           const int k = __ldg(o.acol + a0 + t);
           bs = __ldg(o.brpt + k);
-          len = __ldg(o.brpt + k + 1) - bs;
+          len = run_len(__ldg(o.brpt + k + 1) - bs);
         }
         // a row of too many products is left before its columns are read
         int total = len;
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
         P += total;
-        if (total < 0 || total > kRunMaxIp || P > kRunMaxIp) {
+        if (P > kRunMaxIp) {
           P = kRunMaxIp + 1;
           break;
         }
@@ -525,9 +525,9 @@ __global__ void __launch_bounds__(256)
           if (t < na) {
             const int k = __ldg(o.acol + a0 + t), k2 = __ldg(o2.acol + a2 + t);
             bs = __ldg(o.brpt + k);
-            len = __ldg(o.brpt + k + 1) - bs;
+            len = run_len(__ldg(o.brpt + k + 1) - bs);
             bs2 = __ldg(o2.brpt + k2);
-            len2 = __ldg(o2.brpt + k2 + 1) - bs2;
+            len2 = run_len(__ldg(o2.brpt + k2 + 1) - bs2);
             diff = len != len2;
           }
           const unsigned some = __ballot_sync(0xffffffffu, len2 > 0);
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(kProgThreads)
     const RunTerm r = run_term(o, a0 + tid, sigma);
     tk[tid] = r.k;
     tbs[tid] = r.bs;
-    tlen[tid] = r.len;
+    tlen[tid] = run_len(r.len);
     tpl[tid] = r.pl;
   }
   __syncthreads();

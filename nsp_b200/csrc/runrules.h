@@ -1,0 +1,22 @@
+// Limits and arithmetic of the row runs (rowrun.cu) that host code can compile
+// and test as well.
+#pragma once
+
+#ifdef __CUDACC__
+#define NSPB_HD __host__ __device__ __forceinline__
+#else
+#define NSPB_HD inline
+#endif
+
+namespace nspb {
+
+constexpr int kRunMaxA = 128;   // A entries of a row in a run
+constexpr int kRunMaxIp = 1536; // products of a row in a run
+
+// A B row's length as the sums over a row's A entries take it: any that is too
+// long for a run by itself counts as just too long, so that the sum over
+// kRunMaxA entries stays far below 2^31 (a row of A may repeat a column, and 32
+// B rows of 2^27 entries add up to zero in 32 bits).
+NSPB_HD int run_len(int len) { return len < kRunMaxIp + 1 ? len : kRunMaxIp + 1; }
+
+}  // namespace nspb

@@ -1,0 +1,46 @@
+"""The limits of the row runs (runrules.h), compiled for the host: what the kernels
+compute in 32 bits against Python's integers, up to the largest operands."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("rules") / "librules.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-pthread", "-shared", "-fPIC",
+                    "-I", os.path.join(ROOT, "nsp_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "native", "run_rules.cpp"), "-o", so], check=True)
+    return C.CDLL(so)
+
+
+def lengths():
+    big = 1 << 27
+    yield [big] * 32 + [5]                      # 2^32 + 5
+    yield [big] * 31 + [big - 3] + [5]
+    yield [(1 << 31) - 1] * 2 + [2 + 7]         # 2^32 + 7
+    yield [1 << 26] * 64 + [1]
+    yield [1 << 30] * 4 + [1536]
+    yield [1536]
+    yield [1537]
+    yield [12] * 128
+    yield [12] * 127 + [13]
+    yield [0] * 128
+    rng = np.random.default_rng(1)
+    for _ in range(300):
+        n = int(rng.integers(1, 129))
+        top = int(2 ** rng.uniform(0, 31)) - 1
+        yield [int(x) for x in rng.integers(0, max(top, 1), n)]
+
+
+def test_products_of_a_row_do_not_wrap(rules):
+    limit = rules.max_ip()
+    for lens in lengths():
+        assert len(lens) <= rules.max_a()
+        got = rules.row_products((C.c_int * len(lens))(*lens), len(lens))
+        assert got == min(sum(lens), limit + 1), lens
