@@ -1465,6 +1465,20 @@ __global__ void __launch_bounds__((RunCfg<CLASS>::WARPS + RunCfg<CLASS>::LOOK) *
     __syncwarp();
     asm volatile("barrier.sync 1, %0;" ::"n"(THREADS) : "memory");
   };
+  // the same barrier, and whether any thread says yes
+  auto meet_any = [](bool yes) {
+    __syncwarp();
+    unsigned any;
+    asm volatile(
+        "{\n .reg .pred p, q;\n"
+        " setp.ne.u32 q, %1, 0;\n"
+        " barrier.red.or.pred p, 1, %2, q;\n"
+        " selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(any)
+        : "r"((unsigned)yes), "n"(THREADS)
+        : "memory");
+    return any != 0;
+  };
   int cur = -1;  // the program in shared memory
   int na = 0, P = 0, n = 0, parts = 1, pstep = 0, w0 = 0, w1 = 0, rg = 0;
   RunSmem<VT> sm(smem_run, 0, 0, 0, 0);
@@ -1474,8 +1488,7 @@ __global__ void __launch_bounds__((RunCfg<CLASS>::WARPS + RunCfg<CLASS>::LOOK) *
     __syncwarp();
     if (!*(volatile int *)&s_lost && !mbar_wait(&s_full, (unsigned)t & 1u)) s_lost = 1;
     const RunTile &tile = s_tile[t & 1];
-    meet();
-    if (*(volatile int *)&s_lost) {  // uniform unless lost just now: every wait is bounded
+    if (run_gives_up([&] { return *(volatile int *)&s_lost != 0; }, meet_any)) {
       if (tid == 0) atomicOr(err, ERR_WAIT);
       break;
     }

@@ -19,4 +19,13 @@ constexpr int kRunMaxIp = 1536; // products of a row in a run
 // B rows of 2^27 entries add up to zero in 32 bits).
 NSPB_HD int run_len(int len) { return len < kRunMaxIp + 1 ? len : kRunMaxIp + 1; }
 
+// Whether a block of k_num_run stops because a wait has run out. A look-up warp
+// or a lane may find that out at any moment, and a warp that stopped alone
+// would leave the others at their next barrier for good: every warp's view of
+// the flag goes into one vote at a barrier, `any`, and all act on its result.
+template <typename Lost, typename Any>
+NSPB_HD bool run_gives_up(Lost &&lost, Any &&any) {
+  return any(lost());
+}
+
 }  // namespace nspb

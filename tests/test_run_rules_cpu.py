@@ -44,3 +44,13 @@ def test_products_of_a_row_do_not_wrap(rules):
         assert len(lens) <= rules.max_a()
         got = rules.row_products((C.c_int * len(lens))(*lens), len(lens))
         assert got == min(sum(lens), limit + 1), lens
+
+
+@pytest.mark.parametrize("warps", [8, 16])
+def test_a_block_gives_up_as_a_whole(rules, warps):
+    """A wait runs out while the warps of a block look at the flag one after the
+    other: all of them stop, or none."""
+    for after in range(-1, warps):
+        assert rules.warps_that_stop(warps, after) in (0, warps), after
+    assert rules.warps_that_stop(warps, warps) == 0
+    assert rules.warps_that_stop(warps, 0) == warps
