@@ -863,6 +863,9 @@ __global__ void __launch_bounds__(kProgThreads)
       return __shfl_sync(0xffffffffu, total, (na - 1) & 31);
     };
     auto fits = [&](int L) {
+      bool near = true;
+      for (int t = lane; t < na; t += 32) near = near && run_step_fits(tpl[t], L);
+      if (!__all_sync(0xffffffffu, near)) return false;
       const long long fixed = run_fixed(n, P) + run_tile(L, n, na, vsz);
       if (fixed > smem) return false;
       return fixed + (long long)layout(L, false) * vsz <= smem;

@@ -26,6 +26,13 @@ int row_products(const int *len, int na) {
   return total;
 }
 
+// Values of a tile's one segment of B as the kernel counts them (32 bits), or -1
+// where its rows may not share a tile.
+int tile_values(int step, int rows, int len) {
+  if (!run_step_fits(step, rows)) return -1;
+  return (int)((unsigned)(rows - 1) * (unsigned)step + (unsigned)len);
+}
+
 // Warps of a block decide whether to give up while the flag is raised between
 // the views of warp `after` and of the next one. Returns how many of them stop.
 int warps_that_stop(int warps, int after) {

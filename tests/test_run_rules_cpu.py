@@ -54,3 +54,21 @@ def test_a_block_gives_up_as_a_whole(rules, warps):
         assert rules.warps_that_stop(warps, after) in (0, warps), after
     assert rules.warps_that_stop(warps, warps) == 0
     assert rules.warps_that_stop(warps, 0) == warps
+
+
+def test_tiles_of_distant_rows_do_not_wrap(rules):
+    """Every distance between rows that a 32-bit row pointer allows: values counted
+    exactly, or refused; nothing is refused that would fit 110 KB of shared memory
+    and the 15 bits that a program word has for it."""
+    rng = np.random.default_rng(2)
+    steps = [1, 3, 27, 128, 32767, 32768, 1 << 24, (1 << 24) + 3, 1 << 25, 1 << 26, (1 << 27) + 3, 1 << 28,
+             1 << 30, (1 << 31) - 1] + [int(2 ** rng.uniform(0, 31)) for _ in range(200)]
+    for step in steps:
+        for rows in range(1, 129):
+            for n in (1, 128):
+                exact = (rows - 1) * step + n
+                got = rules.tile_values(step, rows, n)
+                if got < 0:
+                    assert exact * 4 > 110000 and step >= 1 << 15, (step, rows)
+                else:
+                    assert got == exact < 1 << 23, (step, rows)
