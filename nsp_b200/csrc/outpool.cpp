@@ -8,10 +8,12 @@
 //
 // What callers rely on stays:
 //  - the block is an allocation of its own (cudaMalloc): cudaFree on it works,
-//    and then it is simply gone. A block is checked against the driver's idea
-//    of its address whenever it is kept, given out again or freed here, so one
-//    that its caller freed as well is never touched; nspb_free of a block that
-//    is kept already is an error, as a second cudaFree was.
+//    and then it is simply gone. The driver numbers every allocation of the
+//    process; a block is kept, given out again or freed here only while its
+//    address still has the number it was allocated with, so one that its caller
+//    freed as well is never touched, also when the address (and the size)
+//    belong to someone else by then. nspb_free of a block that is kept already
+//    is an error, as a second cudaFree was.
 //  - nspb_free waits for the device like cudaFree, so that work in flight on
 //    any stream has read a block before it is given out again; where the wait
 //    is not possible (a capture in progress) the block goes to cudaFree.
@@ -42,13 +44,14 @@ constexpr size_t kMaxLive = 4096;
 struct Block {
   void *p;
   size_t bytes;
+  unsigned long long id;  // the driver's number of the allocation
 };
 
 struct Pool {
   std::mutex mu;
-  std::vector<Block> kept;                     // oldest first
+  std::vector<Block> kept;                   // oldest first
   size_t kept_bytes = 0;
-  std::unordered_map<void *, size_t> live;     // handed out and not seen by nspb_free
+  std::unordered_map<void *, Block> live;    // handed out and not seen by nspb_free
 };
 
 // Never destroyed: outputs may outlive the library's static objects.
@@ -66,39 +69,36 @@ int current_device() {
   return dev >= 0 && dev < kMaxDevices ? dev : -1;
 }
 
-// Whether p is still the start of an allocation of this many bytes on device dev.
-bool still_block(void *p, size_t bytes, int dev) {
-  using Range = CUresult (*)(CUdeviceptr *, size_t *, CUdeviceptr);
-  static const Range range = [] {
+// The number of the allocation that p lies in (unique in the process, and
+// readable from a thread that has no context yet); 0 when it lies in none.
+unsigned long long allocation_id(void *p) {
+  using Attribute = CUresult (*)(void *, CUpointer_attribute, CUdeviceptr);
+  static const Attribute attribute = [] {
     void *fn = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+    if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &q) != cudaSuccess ||
         q != cudaDriverEntryPointSuccess) {
       cudaGetLastError();
       fn = nullptr;
     }
-    return reinterpret_cast<Range>(fn);
+    return reinterpret_cast<Attribute>(fn);
   }();
-  if (!range) return false;
-  cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  if (at.type != cudaMemoryTypeDevice || at.device != dev) return false;
-  CUdeviceptr base = 0;
-  size_t size = 0;
-  return range(&base, &size, reinterpret_cast<CUdeviceptr>(p)) == CUDA_SUCCESS &&
-         base == reinterpret_cast<CUdeviceptr>(p) && size == bytes;
+  unsigned long long id = 0;
+  if (!attribute || attribute(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID,
+                              reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS)
+    return 0;
+  return id;
 }
 
-cudaError_t drop(Pool &pl, int dev, size_t down_to) {
+bool still_block(const Block &b) { return b.id != 0 && allocation_id(b.p) == b.id; }
+
+cudaError_t drop(Pool &pl, size_t down_to) {
   cudaError_t first = cudaSuccess;
   while (!pl.kept.empty() && pl.kept_bytes > down_to) {
     const Block b = pl.kept.front();
     pl.kept.erase(pl.kept.begin());
     pl.kept_bytes -= b.bytes;
-    const cudaError_t e = still_block(b.p, b.bytes, dev) ? cudaFree(b.p) : cudaSuccess;
+    const cudaError_t e = still_block(b) ? cudaFree(b.p) : cudaSuccess;
     if (first == cudaSuccess) first = e;
   }
   return first;
@@ -122,9 +122,9 @@ int alloc_out(void **p, size_t bytes) {
       const Block b = *best;
       pl.kept_bytes -= b.bytes;
       pl.kept.erase(best);
-      if (!still_block(b.p, b.bytes, dev)) continue;  // its caller freed it as well
+      if (!still_block(b)) continue;  // its caller freed it as well
       *p = b.p;
-      pl.live[b.p] = b.bytes;
+      pl.live[b.p] = b;
       return NSPB_OK;
     }
   }
@@ -133,7 +133,7 @@ int alloc_out(void **p, size_t bytes) {
     cudaGetLastError();
     Pool &pl = pool_of(dev);
     std::lock_guard<std::mutex> lock(pl.mu);
-    drop(pl, dev, 0);
+    drop(pl, 0);
     e = cudaMalloc(p, bytes);
   }
   if (e != cudaSuccess) {
@@ -146,7 +146,7 @@ int alloc_out(void **p, size_t bytes) {
     std::lock_guard<std::mutex> lock(pl.mu);
     // blocks that went to cudaFree directly leave entries behind
     if (pl.live.size() >= kMaxLive) pl.live.clear();
-    pl.live[*p] = bytes;
+    pl.live[*p] = Block{*p, bytes, allocation_id(*p)};
   }
   return NSPB_OK;
 }
@@ -157,21 +157,21 @@ static int keep_out(void *p) {
   const int dev = current_device();
   if (dev < 0) return 0;
   Pool &pl = pool_of(dev);
-  size_t bytes;
+  Block b;
   {
     std::lock_guard<std::mutex> lock(pl.mu);
     auto it = pl.live.find(p);
     if (it == pl.live.end()) {
-      for (const Block &b : pl.kept)
-        if (b.p == p && still_block(p, b.bytes, dev)) return -1;
+      for (const Block &k : pl.kept)
+        if (k.p == p && still_block(k)) return -1;
       return 0;
     }
-    bytes = it->second;
+    b = it->second;
     pl.live.erase(it);
   }
   const size_t cap = dev_info().total_mem / 16;
-  if (bytes > cap || !still_block(p, bytes, dev)) return 0;
-  if (bytes >= kAskFree) {
+  if (b.bytes > cap || !still_block(b)) return 0;
+  if (b.bytes >= kAskFree) {
     size_t free_b = 0, total = 0;
     if (cudaMemGetInfo(&free_b, &total) != cudaSuccess || free_b < total / 4) {
       cudaGetLastError();
@@ -183,9 +183,9 @@ static int keep_out(void *p) {
     return 0;
   }
   std::lock_guard<std::mutex> lock(pl.mu);
-  drop(pl, dev, cap - bytes);
-  pl.kept.push_back(Block{p, bytes});
-  pl.kept_bytes += bytes;
+  drop(pl, cap - b.bytes);
+  pl.kept.push_back(b);
+  pl.kept_bytes += b.bytes;
   return 1;
 }
 
@@ -211,7 +211,7 @@ extern "C" int nspb_trim(void) {
   if (dev < 0) return NSPB_ERR_NO_DEVICE;
   Pool &pl = pool_of(dev);
   std::lock_guard<std::mutex> lock(pl.mu);
-  const cudaError_t e = drop(pl, dev, 0);
+  const cudaError_t e = drop(pl, 0);
   if (e != cudaSuccess) {
     g_last_cuda = (int)e;
     cudaGetLastError();
