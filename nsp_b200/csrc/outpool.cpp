@@ -15,8 +15,12 @@
 //    belong to someone else by then. nspb_free of a block that is kept already
 //    is an error, as a second cudaFree was.
 //  - nspb_free waits for the device like cudaFree, so that work in flight on
-//    any stream has read a block before it is given out again; where the wait
-//    is not possible (a capture in progress) the block goes to cudaFree.
+//    any stream has read a block before it is given out again, and where
+//    cudaFree may be called it may be: it waits by freeing a block of 512 bytes
+//    (5 us). cudaDeviceSynchronize would end every capture in progress on the
+//    device, also those of other threads and relaxed ones, a plan's for
+//    instance. Where cudaFree is not allowed (a global capture), the error is
+//    cudaFree's own.
 // The blocks kept on a device hold at most a sixteenth of its memory, only
 // while a quarter of it is free, the longest unused leave first, and all of
 // them when an allocation fails; nspb_trim gives them back at any time.
@@ -91,6 +95,14 @@ unsigned long long allocation_id(void *p) {
 }
 
 bool still_block(const Block &b) { return b.id != 0 && allocation_id(b.p) == b.id; }
+
+// Waits until the device has done all work given to it, as cudaFree does.
+bool wait_for_device() {
+  void *p = nullptr;
+  if (cudaMalloc(&p, kGrain) == cudaSuccess && cudaFree(p) == cudaSuccess) return true;
+  cudaGetLastError();
+  return false;
+}
 
 cudaError_t drop(Pool &pl, size_t down_to) {
   cudaError_t first = cudaSuccess;
@@ -178,10 +190,7 @@ static int keep_out(void *p) {
       return 0;
     }
   }
-  if (cudaDeviceSynchronize() != cudaSuccess) {  // a capture in progress, or an earlier fault
-    cudaGetLastError();
-    return 0;
-  }
+  if (!wait_for_device()) return 0;  // a capture in progress, or an earlier fault
   std::lock_guard<std::mutex> lock(pl.mu);
   drop(pl, cap - b.bytes);
   pl.kept.push_back(b);

@@ -22,6 +22,16 @@ std::map<size_t, Alloc> mem;  // by address
 unsigned long long next_id = 1;
 size_t capacity = (size_t)180 << 30;
 thread_local bool no_context = false;
+int capture = 0;           // 0 none, 1 another thread's thread-local or a relaxed one, 2 global
+bool capture_ends = false; // a call that is not allowed in it was made
+int waits = 0;             // calls that waited for the device
+
+// A call that a capture of this kind (and any stricter one) does not allow.
+bool forbidden(int from) {
+  if (capture < from) return false;
+  capture_ends = true;
+  return true;
+}
 
 size_t used() {
   size_t sum = 0;
@@ -87,14 +97,21 @@ cudaError_t cudaGetDevice(int *dev) {
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 cudaError_t cudaMalloc(void **p, size_t bytes) {
   no_context = false;
+  if (forbidden(2)) return cudaErrorStreamCaptureUnsupported;
   return take(p, bytes);
 }
 cudaError_t cudaFree(void *p) {
   std::lock_guard<std::recursive_mutex> lock(mu);
   no_context = false;
+  if (forbidden(2)) return cudaErrorStreamCaptureUnsupported;
+  ++waits;
   return mem.erase(reinterpret_cast<size_t>(p)) ? cudaSuccess : cudaErrorInvalidValue;
 }
-cudaError_t cudaDeviceSynchronize(void) { return cudaSuccess; }
+cudaError_t cudaDeviceSynchronize(void) {
+  if (forbidden(1)) return cudaErrorStreamCaptureUnsupported;
+  ++waits;
+  return cudaSuccess;
+}
 cudaError_t cudaMemGetInfo(size_t *free_b, size_t *total) {
   std::lock_guard<std::recursive_mutex> lock(mu);
   *total = capacity;
@@ -128,6 +145,12 @@ size_t fake_used(void) {
   return used();
 }
 void fake_capacity(size_t bytes) { capacity = bytes; }
+void fake_capture(int kind) {
+  capture = kind;
+  capture_ends = false;
+}
+int fake_capture_ends(void) { return capture_ends; }
+int fake_waits(void) { return waits; }
 void fake_no_context(void) { no_context = true; }
 int fake_alloc_out(void **p, size_t bytes) { return nspb::alloc_out(p, bytes); }
 }

@@ -111,3 +111,23 @@ def test_a_thread_without_a_context(pool, use):
     else:
         assert out(pool, 40 * MB) == p
         assert pool.nspb_free(p) == 0
+
+
+def test_a_capture_elsewhere_goes_on(pool):
+    """nspb_free during another thread's thread-local capture, or a relaxed one: allowed, as
+    cudaFree is, and the device is waited for before the block can be given out again."""
+    p = out(pool, 40 * MB)
+    pool.fake_capture(1)
+    before = pool.fake_waits()
+    assert pool.nspb_free(p) == 0
+    assert pool.fake_waits() > before
+    assert not pool.fake_capture_ends()
+    pool.fake_capture(0)
+
+
+def test_a_global_capture_refuses(pool):
+    p = out(pool, 40 * MB)
+    pool.fake_capture(2)
+    assert pool.nspb_free(p) != 0
+    pool.fake_capture(0)
+    assert pool.nspb_free(p) == 0

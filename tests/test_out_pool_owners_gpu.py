@@ -60,3 +60,40 @@ def test_trim_in_a_new_thread_gives_the_memory_back(cuda):
     t.join()
     assert r == [0]
     assert torch.cuda.mem_get_info()[0] - kept >= 32 << 20
+
+
+@pytest.mark.parametrize("mode", [1, 2])  # another thread's thread-local capture, a relaxed one
+def test_captures_go_on(cuda, mode):
+    """An output is freed while another thread captures a stream: the capture is whole."""
+    A = nb.gen.stencil(20, npts=27).to_device()
+    c = product(A)
+    s, g = C.c_void_p(), C.c_void_p()
+    assert rt.cudaStreamCreateWithFlags(C.byref(s), 1) == 0
+    assert rt.cudaStreamBeginCapture(s, mode) == 0
+    r = []
+    t = threading.Thread(target=lambda: r.extend(lib.nspb_free(p) for p in ptrs(c)))
+    t.start()
+    t.join()
+    end = rt.cudaStreamEndCapture(s, C.byref(g))
+    rt.cudaGetLastError()
+    assert r == [0, 0, 0] and end == 0
+    assert rt.cudaGraphDestroy(g) == 0 and rt.cudaStreamDestroy(s) == 0
+
+
+def test_plans_are_made_while_outputs_are_freed(cuda):
+    A = nb.gen.stencil(12, npts=27).to_device()
+    stop, made = threading.Event(), []
+
+    def products():
+        while not stop.is_set():
+            for p in ptrs(product(A)):
+                made.append(lib.nspb_free(p))
+    t = threading.Thread(target=products)
+    t.start()
+    try:
+        for _ in range(60):
+            nb.Plan([A], [A]).execute()
+    finally:
+        stop.set()
+        t.join()
+    assert made and not any(made)
