@@ -405,13 +405,7 @@ int plan_fail(cudaError_t e) {
 
 template <typename T>
 int dev_alloc(T **p, size_t count) {
-  cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), std::max<size_t>(count, 1) * sizeof(T));
-  if (e != cudaSuccess) {
-    g_last_cuda = (int)e;
-    cudaGetLastError();
-    return NSPB_ERR_ALLOC;
-  }
-  return NSPB_OK;
+  return device_alloc(reinterpret_cast<void **>(p), std::max<size_t>(count, 1) * sizeof(T));
 }
 
 // The numeric phase of a group as launched on every execution: counters

@@ -1,4 +1,5 @@
-// Blocks for the outputs that the library allocates, kept between calls.
+// The library's device memory: blocks for the outputs that it allocates, kept
+// between calls, and its scratch.
 //
 // A product that allocates C pays cudaMalloc for it, and its caller cudaFree:
 // for C of 555 MB that was 2.3 ms of a 3.9 ms call whose kernels take 1.5 ms,
@@ -23,7 +24,9 @@
 //    cudaFree's own.
 // The blocks kept on a device hold at most a sixteenth of its memory, only
 // while a quarter of it is free, the longest unused leave first, and all of
-// them when an allocation fails; nspb_trim gives them back at any time.
+// them when an allocation of the library fails, for an output, for scratch or
+// for a plan, which is then tried again: what a call could have while nspb_free
+// gave every block back, it still has. nspb_trim gives them back at any time.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -118,6 +121,67 @@ cudaError_t drop(Pool &pl, size_t down_to) {
 
 }  // namespace
 
+// cudaFree of every block kept on the current device; whether there was one.
+static bool give_back() {
+  const int dev = current_device();
+  if (dev < 0) return false;
+  Pool &pl = pool_of(dev);
+  std::lock_guard<std::mutex> lock(pl.mu);
+  const bool any = !pl.kept.empty();
+  drop(pl, 0);
+  return any;
+}
+
+// Runs an allocation, and again without the kept blocks if there is no memory.
+template <typename F>
+static int allocate(F &&f) {
+  cudaError_t e = f();
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (give_back()) e = f();
+  }
+  if (e == cudaSuccess) return NSPB_OK;
+  g_last_cuda = (int)e;
+  cudaGetLastError();
+  return NSPB_ERR_ALLOC;
+}
+
+int device_alloc(void **p, size_t bytes) {
+  return allocate([&] { return cudaMalloc(p, bytes); });
+}
+
+// Library-owned stream-ordered pool per device; freed blocks stay cached.
+static cudaMemPool_t scratch_pool() {
+  static std::mutex mu;
+  static cudaMemPool_t pools[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) dev = 0;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
+    uint64_t keep = UINT64_MAX;
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    pools[dev] = p;
+  }
+  return pools[dev];
+}
+
+int scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
+  cudaMemPool_t pool = scratch_pool();
+  if (!pool) return NSPB_ERR_ALLOC;
+  return allocate([&] { return cudaMallocFromPoolAsync(p, bytes < 256 ? 256 : bytes, pool, s); });
+}
+
+void scratch_free(void *p, cudaStream_t s) {
+  if (p) cudaFreeAsync(p, s);
+}
+
 int alloc_out(void **p, size_t bytes) {
   bytes = (std::max<size_t>(bytes, 4) + kGrain - 1) / kGrain * kGrain;
   const int dev = current_device();
@@ -140,19 +204,8 @@ int alloc_out(void **p, size_t bytes) {
       return NSPB_OK;
     }
   }
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e == cudaErrorMemoryAllocation && dev >= 0) {
-    cudaGetLastError();
-    Pool &pl = pool_of(dev);
-    std::lock_guard<std::mutex> lock(pl.mu);
-    drop(pl, 0);
-    e = cudaMalloc(p, bytes);
-  }
-  if (e != cudaSuccess) {
-    g_last_cuda = (int)e;
-    cudaGetLastError();
-    return NSPB_ERR_ALLOC;
-  }
+  const int st = device_alloc(p, bytes);
+  if (st) return st;
   if (dev >= 0) {
     Pool &pl = pool_of(dev);
     std::lock_guard<std::mutex> lock(pl.mu);

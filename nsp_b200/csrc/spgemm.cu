@@ -48,44 +48,6 @@ const DevInfo &dev_info() {
   return d;
 }
 
-// Library-owned stream-ordered pool per device; freed blocks stay cached.
-static cudaMemPool_t scratch_pool() {
-  static std::mutex mu;
-  static cudaMemPool_t pools[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!pools[dev]) {
-    cudaMemPoolProps props = {};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t p = nullptr;
-    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
-    uint64_t keep = UINT64_MAX;
-    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    pools[dev] = p;
-  }
-  return pools[dev];
-}
-
-int scratch_alloc(void **p, size_t bytes, cudaStream_t s) {
-  cudaMemPool_t pool = scratch_pool();
-  if (!pool) return NSPB_ERR_ALLOC;
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes < 256 ? 256 : bytes, pool, s);
-  if (e != cudaSuccess) {
-    g_last_cuda = (int)e;
-    cudaGetLastError();
-    return NSPB_ERR_ALLOC;
-  }
-  return NSPB_OK;
-}
-
-void scratch_free(void *p, cudaStream_t s) {
-  if (p) cudaFreeAsync(p, s);
-}
-
 // Pinned staging for the two small device->host reads of a call.
 HostStage *host_stage() {
   struct Holder {

@@ -44,9 +44,11 @@ struct HostStage {
 };
 
 HostStage *host_stage();
+// outpool.cpp
 int scratch_alloc(void **p, size_t bytes, cudaStream_t s);
 void scratch_free(void *p, cudaStream_t s);
-int alloc_out(void **p, size_t bytes);
+int device_alloc(void **p, size_t bytes);  // cudaMalloc
+int alloc_out(void **p, size_t bytes);     // an output, released with nspb_free
 
 struct Call {
   nspb_opts opts{};

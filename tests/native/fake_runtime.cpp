@@ -112,6 +112,18 @@ cudaError_t cudaDeviceSynchronize(void) {
   ++waits;
   return cudaSuccess;
 }
+cudaError_t cudaMemPoolCreate(cudaMemPool_t *pool, const cudaMemPoolProps *) {
+  *pool = reinterpret_cast<cudaMemPool_t>(&mem);
+  return cudaSuccess;
+}
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
+cudaError_t cudaMallocFromPoolAsync(void **p, size_t bytes, cudaMemPool_t, cudaStream_t) {
+  return take(p, bytes);
+}
+cudaError_t cudaFreeAsync(void *p, cudaStream_t) {
+  std::lock_guard<std::recursive_mutex> lock(mu);
+  return mem.erase(reinterpret_cast<size_t>(p)) ? cudaSuccess : cudaErrorInvalidValue;
+}
 cudaError_t cudaMemGetInfo(size_t *free_b, size_t *total) {
   std::lock_guard<std::recursive_mutex> lock(mu);
   *total = capacity;
@@ -152,5 +164,7 @@ void fake_capture(int kind) {
 int fake_capture_ends(void) { return capture_ends; }
 int fake_waits(void) { return waits; }
 void fake_no_context(void) { no_context = true; }
+int fake_scratch(void **p, size_t bytes) { return nspb::scratch_alloc(p, bytes, nullptr); }
+int fake_device(void **p, size_t bytes) { return nspb::device_alloc(p, bytes); }
 int fake_alloc_out(void **p, size_t bytes) { return nspb::alloc_out(p, bytes); }
 }

@@ -30,7 +30,8 @@ def pool(built):
     lib.fake_malloc.argtypes = lib.fake_capacity.argtypes = [C.c_size_t]
     lib.fake_free.argtypes = lib.nspb_free.argtypes = [C.c_void_p]
     lib.fake_used.restype = C.c_size_t
-    lib.fake_alloc_out.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
+    for f in (lib.fake_scratch, lib.fake_device, lib.fake_alloc_out):
+        f.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
     lib.fake_capacity(180 << 30)
     assert lib.nspb_trim() == 0 and lib.fake_used() == 0
     yield lib
@@ -130,4 +131,21 @@ def test_a_global_capture_refuses(pool):
     pool.fake_capture(2)
     assert pool.nspb_free(p) != 0
     pool.fake_capture(0)
+    assert pool.nspb_free(p) == 0
+
+
+@pytest.mark.parametrize("kind", ["fake_scratch", "fake_device", "fake_alloc_out"])
+def test_kept_blocks_leave_when_memory_is_short(pool, kind):
+    """Scratch, a plan's arrays and outputs get the memory of the kept blocks before
+    an allocation fails; past that it still fails."""
+    pool.fake_capacity(1600 * MB)
+    ps = [out(pool, 30 * MB) for _ in range(3)]
+    for p in ps:
+        assert pool.nspb_free(p) == 0
+    assert pool.fake_used() == 90 * MB
+    p = C.c_void_p()
+    assert getattr(pool, kind)(C.byref(p), 1550 * MB) == 0
+    assert pool.fake_used() == 1550 * MB
+    q = C.c_void_p()
+    assert getattr(pool, kind)(C.byref(q), 100 * MB) != 0
     assert pool.nspb_free(p) == 0
