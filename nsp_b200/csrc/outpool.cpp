@@ -32,6 +32,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <new>
 #include <unordered_map>
 #include <vector>
 
@@ -61,9 +62,27 @@ struct Pool {
   std::unordered_map<void *, Block> live;    // handed out and not seen by nspb_free
 };
 
+// Bookkeeping that finds no host memory: the block is not kept (or not known as
+// an output, so that nspb_free takes it to cudaFree). No exception leaves here,
+// the callers are C functions.
+template <typename F>
+bool noted(F &&f) noexcept {
+  try {
+    f();
+    return true;
+  } catch (...) {
+    return false;
+  }
+}
+
 // Never destroyed: outputs may outlive the library's static objects.
 Pool &pool_of(int dev) {
-  static Pool *pools = new Pool[kMaxDevices];
+  alignas(Pool) static unsigned char room[sizeof(Pool) * kMaxDevices];
+  static Pool *pools = [] {
+    Pool *first = reinterpret_cast<Pool *>(room);
+    for (int i = 0; i < kMaxDevices; ++i) new (first + i) Pool;
+    return first;
+  }();
   return pools[dev];
 }
 
@@ -200,7 +219,7 @@ int alloc_out(void **p, size_t bytes) {
       pl.kept.erase(best);
       if (!still_block(b)) continue;  // its caller freed it as well
       *p = b.p;
-      pl.live[b.p] = b;
+      noted([&] { pl.live[b.p] = b; });
       return NSPB_OK;
     }
   }
@@ -211,7 +230,7 @@ int alloc_out(void **p, size_t bytes) {
     std::lock_guard<std::mutex> lock(pl.mu);
     // blocks that went to cudaFree directly leave entries behind
     if (pl.live.size() >= kMaxLive) pl.live.clear();
-    pl.live[*p] = Block{*p, bytes, allocation_id(*p)};
+    noted([&] { pl.live[*p] = Block{*p, bytes, allocation_id(*p)}; });
   }
   return NSPB_OK;
 }
@@ -246,7 +265,7 @@ static int keep_out(void *p) {
   if (!wait_for_device()) return 0;  // a capture in progress, or an earlier fault
   std::lock_guard<std::mutex> lock(pl.mu);
   drop(pl, cap - b.bytes);
-  pl.kept.push_back(b);
+  if (!noted([&] { pl.kept.push_back(b); })) return 0;
   pl.kept_bytes += b.bytes;
   return 1;
 }

@@ -4,12 +4,26 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 
 #include "internal.h"
 #include "spgemm_host.h"
+
+namespace {
+bool no_host_memory = false;
+}
+// what outpool.cpp's containers allocate with
+void *operator new(size_t bytes) {
+  if (no_host_memory) throw std::bad_alloc();
+  if (void *p = std::malloc(bytes)) return p;
+  throw std::bad_alloc();
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 namespace {
 
@@ -47,7 +61,10 @@ cudaError_t take(void **p, size_t bytes) {
     if (a.first - at >= bytes) break;
     at = a.first + a.second.bytes;
   }
+  const bool was = no_host_memory;  // the fake's own books are another matter
+  no_host_memory = false;
   mem[at] = Alloc{bytes, next_id++};
+  no_host_memory = was;
   *p = reinterpret_cast<void *>(at);
   return cudaSuccess;
 }
@@ -163,6 +180,7 @@ void fake_capture(int kind) {
 }
 int fake_capture_ends(void) { return capture_ends; }
 int fake_waits(void) { return waits; }
+void fake_no_host_memory(int yes) { no_host_memory = yes; }
 void fake_no_context(void) { no_context = true; }
 int fake_scratch(void **p, size_t bytes) { return nspb::scratch_alloc(p, bytes, nullptr); }
 int fake_device(void **p, size_t bytes) { return nspb::device_alloc(p, bytes); }

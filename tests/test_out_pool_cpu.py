@@ -3,6 +3,7 @@ that only hands out addresses: whose memory a block is, and from which thread.""
 import ctypes as C
 import os
 import subprocess
+import sys
 import threading
 
 import pytest
@@ -149,3 +150,33 @@ def test_kept_blocks_leave_when_memory_is_short(pool, kind):
     q = C.c_void_p()
     assert getattr(pool, kind)(C.byref(q), 100 * MB) != 0
     assert pool.nspb_free(p) == 0
+
+
+HOST_MEMORY = """
+import ctypes as C, sys
+lib = C.CDLL(sys.argv[1])
+lib.nspb_free.argtypes = [C.c_void_p]
+lib.fake_alloc_out.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
+lib.fake_used.restype = C.c_size_t
+step, p = sys.argv[2], C.c_void_p()
+if step == "first":
+    lib.fake_no_host_memory(1)
+assert lib.fake_alloc_out(C.byref(p), 40 << 20) == 0
+if step == "again":
+    assert lib.nspb_free(p) == 0
+    lib.fake_no_host_memory(1)
+    q = C.c_void_p()
+    assert lib.fake_alloc_out(C.byref(q), 40 << 20) == 0 and q.value == p.value
+if step == "free":
+    lib.fake_no_host_memory(1)
+assert lib.nspb_free(p) == 0
+lib.fake_no_host_memory(0)
+assert lib.nspb_trim() == 0
+assert lib.fake_used() == 0
+"""
+
+
+@pytest.mark.parametrize("step", ["first", "again", "free"])
+def test_no_host_memory_for_the_books(built, step):
+    """An exception of the containers stays inside: the call works, the block is not kept."""
+    subprocess.run([sys.executable, "-c", HOST_MEMORY, built, step], check=True)
