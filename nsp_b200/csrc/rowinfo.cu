@@ -83,14 +83,75 @@ cudaError_t launch_check_sorted_table(const Operands<void> *ops, int nprod, int 
 // a power-law row of 10^4 entries does not leave one lane group walking it.
 constexpr int kRowinfoLong = 1024;
 
+// Counts and bins, GA lanes a row: where no runs are wanted, for rows of more
+// than kInfoSerial entries on average and for fewer than kGroupInfoRows rows.
+// The tiles of k_rowinfo keep few threads busy there (products of every row,
+// this kernel and the tiles: 50,000 rows of 700 entries 132 and 289 us, 2000 of
+// 300 39 and 52, 8000 of 27 39 and 45; 33,000 of 27 46 and 40 the other way).
+constexpr int kInfoSerial = 64;
+constexpr int kGroupInfoRows = 10000;
+template <int GA, bool MULTI>
+__global__ void __launch_bounds__(256)
+    k_rowinfo_group(const ProdTable<void> src, int n, const BinLimits lim,
+              int *__restrict__ row_nz, int64_t *__restrict__ row_ip,
+              int *__restrict__ sym_counts,
+              unsigned long long *__restrict__ total_ip, int *__restrict__ flags,
+              int *__restrict__ long_list, int *__restrict__ long_count) {
+  // With flags (B is A): the order of every row read here is checked too,
+  // which is the B check of launch_check_sorted without a second read.
+  // persistent grid: bin counts and the total accumulate in shared memory and
+  // reach global memory once per block (one block per few rows made every
+  // block add into the same dozen counters)
+  __shared__ int hist[kSymBins];
+  __shared__ unsigned long long s_total;
+  if (threadIdx.x < kSymBins) hist[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_total = 0ull;
+  __syncthreads();
+  auto tile = cg::tiled_partition<GA>(cg::this_thread_block());
+  const int lane = tile.thread_rank();
+  constexpr int kGroups = 256 / GA;
+  unsigned long long my_total = 0;
+  int bad = 0;
+  for (int row = blockIdx.x * kGroups + (int)threadIdx.x / GA; row < n;
+       row += gridDim.x * kGroups) {
+    Operands<void> o;
+    const int lr = prod_row<MULTI>(src, row, o);
+    const int a0 = o.arpt[lr], a1 = o.arpt[lr + 1];
+    if (long_list && a1 - a0 > kRowinfoLong) {  // left to k_rowinfo_long
+      if (lane == 0) long_list[atomicAdd(long_count, 1)] = row;
+      continue;
+    }
+    long long ip = 0;
+    for (int j = a0 + lane; j < a1; j += GA) {
+      const int k = ld_stream(o.acol + j);
+      ip += o.brpt[k + 1] - o.brpt[k];
+      // each entry against its predecessor, read directly: no dependence
+      // between rounds, so long rows keep their loads in flight
+      if (flags && j > a0 && k <= __ldg(o.acol + j - 1)) bad = 1;
+    }
+    ip = cg::reduce(tile, ip, cg::plus<long long>());
+    if (lane == 0) {
+      const int ub = (int)(ip < (long long)o.ncols ? ip : (long long)o.ncols);
+      row_nz[row] = ub;
+      if (row_ip) row_ip[row] = ip;
+      if (ub > 0) atomicAdd(&hist[sym_bin(ub, lim)], 1);
+      my_total += (unsigned long long)ip;
+    }
+  }
+  if (lane == 0 && my_total) atomicAdd(&s_total, my_total);
+  if (__syncthreads_or(bad) && flags && threadIdx.x == 0) atomicOr(flags, B_UNSORTED);
+  if (threadIdx.x < kSymBins && hist[threadIdx.x])
+    atomicAdd(&sym_counts[threadIdx.x], hist[threadIdx.x]);
+  if (threadIdx.x == 0 && s_total) atomicAdd(total_ip, s_total);
+}
+
 // Counts, bins and, where runs are wanted, the links between rows: a thread a
 // row over columns staged in shared memory (common.cuh). On structured
 // operands the threads of a warp then gather neighbouring entries of B's row
 // pointer; a group of lanes a row waited for pointer, columns and gather in
 // turn (370 us on the 27-point 128^3 stencil, 150 us on the power-law 1M
-// matrix). Rows of more than kInfoSerial entries are left to the whole warp,
+// matrix). Rows of more than kInfoSerial entries are left to whole warps,
 // those of more than kRowinfoLong to k_rowinfo_long.
-constexpr int kInfoSerial = 64;
 
 template <bool MULTI>
 __global__ void __launch_bounds__(kTileThreads)
@@ -127,6 +188,9 @@ __global__ void __launch_bounds__(kTileThreads)
   __shared__ unsigned long long s_total;
   __shared__ int cols[kTileWords];
   __shared__ int rp[kTileThreads + kMaxLag + 1];  // row starts from three rows before the tile
+  __shared__ short s_far[kTileThreads];           // rows left to a warp
+  __shared__ long long s_sum[kTileThreads];       // and their products
+  __shared__ int s_nfar;
   if (threadIdx.x < kSymBins) hist[threadIdx.x] = 0;
   if (threadIdx.x == 0) s_total = 0ull;
   __syncthreads();
@@ -243,29 +307,41 @@ __global__ void __launch_bounds__(kTileThreads)
         }
       }
       if (flags) bad |= wrong;
-      // longer rows, a warp a row
-      unsigned todo = __ballot_sync(0xffffffffu, na > kInfoSerial && !code && !listed);
-      while (todo) {
-        const int w = __ffs(todo) - 1;
-        todo &= todo - 1u;
-        const int b0 = __shfl_sync(0xffffffffu, a0, w), b1 = __shfl_sync(0xffffffffu, a1, w);
-        const int *acol = o.acol, *brpt = o.brpt;
-        if (MULTI && split) {
-          acol = reinterpret_cast<const int *>(
-              __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(acol), w));
-          brpt = reinterpret_cast<const int *>(
-              __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(brpt), w));
-        }
-        auto at = [&](int j) { return MULTI && split ? __ldg(acol + j) : col(j); };
-        long long sum = 0;
-        for (int j = b0 + lane; j < b1; j += 32) {
-          const int k = at(j);
-          sum += __ldg(brpt + k + 1) - __ldg(brpt + k);
-          if (flags) bad |= j > b0 && k <= at(j - 1);
-        }
+      // longer rows, a warp a row, all warps sharing the tile's (each warp left
+      // to its own 32 rows: 60,000 rows of 70 entries 90 us, 45 now)
+      const bool far = na > kInfoSerial && !code && !listed;
+      if (__syncthreads_or(far)) {
+        if (threadIdx.x == 0) s_nfar = 0;
+        __syncthreads();
+        if (far) s_far[atomicAdd(&s_nfar, 1)] = (short)q;
+        __syncthreads();
+        for (int i = threadIdx.x >> 5; i < s_nfar; i += kTileThreads / 32) {
+          const int w = s_far[i];
+          int b0, b1;
+          Operands<void> ow;
+          if (MULTI && split) {
+            const int lw = prod_row<MULTI>(src, r0 + w, ow);
+            b0 = __ldg(ow.arpt + lw);
+            b1 = __ldg(ow.arpt + lw + 1);
+          } else {
+            ow = o;
+            b0 = rp[w + kMaxLag];
+            b1 = rp[w + kMaxLag + 1];
+          }
+          auto at = [&](int j) { return MULTI && split ? __ldg(ow.acol + j) : col(j); };
+          long long sum = 0;
+#pragma unroll 4
+          for (int j = b0 + lane; j < b1; j += 32) {
+            const int k = at(j);
+            sum += __ldg(ow.brpt + k + 1) - __ldg(ow.brpt + k);
+            if (flags) bad |= j > b0 && k <= at(j - 1);
+          }
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-        if (lane == w) ip = sum;
+          for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+          if (lane == 0) s_sum[w] = sum;
+        }
+        __syncthreads();
+        if (far) ip = s_sum[q];
       }
       if (q >= nr) return;
       if (listed) {
@@ -358,13 +434,33 @@ cudaError_t launch_rowinfo(const ProdTable<void> &t, int n, int64_t a_nnz, const
                            int *long_count, const RunScan &runs, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   const double avg = (double)a_nnz / (double)n;
-  const int tile = tile_rows(avg);
-  const int grid = (int)std::min<int64_t>(((int64_t)n + tile - 1) / tile,
-                                          (int64_t)dev_info().sms * 6);
   const bool multi = t.prod_of_row != nullptr;
-  auto kern = multi ? k_rowinfo<true> : k_rowinfo<false>;
-  kern<<<grid, kTileThreads, 0, s>>>(t, n, tile, lim, row_nz, row_ip, sym_counts, total_ip, flags,
-                                     long_list, long_count, runs);
+  if (!runs.codes && (n < kGroupInfoRows || avg > kInfoSerial)) {
+    const int ga = avg > 24.0 ? 32 : avg > 12.0 ? 16 : avg > 6.0 ? 8 : 4;
+    const int grid = (int)std::min<int64_t>(((int64_t)n * ga + 255) / 256,
+                                            (int64_t)dev_info().sms * 8);
+#define NSPB_RI(GA)                                                                        \
+  (multi ? k_rowinfo_group<GA, true><<<grid, 256, 0, s>>>(t, n, lim, row_nz, row_ip,       \
+                                                          sym_counts, total_ip, flags,     \
+                                                          long_list, long_count)           \
+         : k_rowinfo_group<GA, false><<<grid, 256, 0, s>>>(t, n, lim, row_nz, row_ip,      \
+                                                           sym_counts, total_ip, flags,    \
+                                                           long_list, long_count))
+    switch (ga) {
+      case 32: NSPB_RI(32); break;
+      case 16: NSPB_RI(16); break;
+      case 8: NSPB_RI(8); break;
+      default: NSPB_RI(4); break;
+    }
+#undef NSPB_RI
+  } else {
+    const int tile = tile_rows(avg);
+    const int grid = (int)std::min<int64_t>(((int64_t)n + tile - 1) / tile,
+                                            (int64_t)dev_info().sms * 6);
+    auto kern = multi ? k_rowinfo<true> : k_rowinfo<false>;
+    kern<<<grid, kTileThreads, 0, s>>>(t, n, tile, lim, row_nz, row_ip, sym_counts, total_ip,
+                                       flags, long_list, long_count, runs);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !long_list) return e;
   auto klong = multi ? k_rowinfo_long<true> : k_rowinfo_long<false>;
