@@ -234,6 +234,25 @@ __device__ __forceinline__ void row_queue_init(RowQueue<THREADS> &rq) {
   if (threadIdx.x == 0) rq.big = 0;
 }
 
+// The same for B rows that are long on average (row_products below).
+template <int THREADS>
+struct RowWarpQueue {
+  int4 q[THREADS];  // one round's A entries: B row start, B row end, A value as two ints
+  int ctr[2][3];    // medium entries, long entries, medium cursor: used in alternate
+                    // rounds, so that one set is cleared while the other is in use
+};
+
+template <int THREADS>
+__device__ __forceinline__ void row_queue_init(RowWarpQueue<THREADS> &rq) {
+  if (threadIdx.x < 6) (&rq.ctr[0][0])[threadIdx.x] = 0;
+}
+
+// LONG: mean B row read above this many entries (k_num_rank and k_sym_wide,
+// k_num_block; measured below).
+constexpr double kLongMean = 56.0, kLongMeanBlock = 128.0;
+template <int THREADS, bool LONG>
+using RowQueueOf = std::conditional_t<LONG, RowWarpQueue<THREADS>, RowQueue<THREADS>>;
+
 // Every product of one A row, spread evenly over a block of THREADS threads
 // whatever the lengths of the B rows it touches (power-law matrices mix rows
 // of one entry with hub rows of 10^4 and more). The A row is taken in rounds
@@ -243,7 +262,7 @@ __device__ __forceinline__ void row_queue_init(RowQueue<THREADS> &rq) {
 // whose places a scan of their lengths gives; warps take pieces of 32
 // consecutive products, lane l the product l of the piece, so that every lane
 // works and neighbours read neighbouring B entries. U pieces' loads are in
-// flight at a time in each warp. ROWPROD_FIG
+// flight at a time in each warp.
 // f(c, a, b) gets the B entry's column, the A value and the B value (values 0
 // when aval / bval are null). Every thread of the block must call this with
 // the same (a0, a1) after a block barrier, and a block barrier must separate
@@ -352,6 +371,95 @@ __device__ __forceinline__ void row_products(const int *__restrict__ acol,
     if (threadIdx.x == 0) rq.big = 0;
     if (jr + THREADS < a1) __syncthreads();
   }
+}
+
+// The same where the B rows are long on average: a B row of at most kRowSmall
+// entries (4 when the round holds fewer than THREADS/4 entries) is walked by its
+// thread, four entries' loads at a time; a longer one by a warp, taken from a
+// shared cursor; one of THREADS entries or more by the whole block.
+// Finding the 32 entries of a piece of the list costs about 50 issue slots,
+// which long rows, filling the lanes by themselves, do not need. Measured, list
+// and this walk, k_num_rank and k_sym_wide: 5000^2 with 700 entries a row 21.1
+// and 10.9 ms; 4000 rows of 150 entries over B rows of 64 entries 1097 and 984
+// us, of 200 over 56 1217 and 1212, of 200 over 48 1101 and 1152; k_num_block:
+// 2000^2 with 140 entries a row 250 and 226 us, 100 a row 165 and 185, 4000^2
+// with 120 a row 732 and 830.
+constexpr int kRowSmall = 16;
+template <int THREADS, int U, typename VT, typename F>
+__device__ __forceinline__ void row_products(const int *__restrict__ acol,
+                                             const VT *__restrict__ aval,
+                                             const int *__restrict__ brpt,
+                                             const int *__restrict__ bcol,
+                                             const VT *__restrict__ bval, int a0, int a1,
+                                             RowWarpQueue<THREADS> &rq, F &&f) {
+  static_assert((THREADS & (THREADS - 1)) == 0, "THREADS must be a power of two");
+  const int lane = threadIdx.x & 31;
+  auto bv = [&](int e) -> double { return bval ? ldv(bval + e) : 0.0; };
+  // entries [e, end) with stride S, two loads in flight per thread
+  auto strided = [&](int e, int end, double a, auto S) {
+    constexpr int kS = decltype(S)::value;
+    for (; e + kS < end; e += 2 * kS) {
+      const int c0 = __ldg(bcol + e), c1 = __ldg(bcol + e + kS);
+      const double b0 = bv(e), b1 = bv(e + kS);
+      f(c0, a, b0);
+      f(c1, a, b1);
+    }
+    if (e < end) f(__ldg(bcol + e), a, bv(e));
+  };
+  int par = 0;
+  for (int jr = a0; jr < a1; jr += THREADS, par ^= 1) {  // uniform across the block
+    const int small_max = min(THREADS, a1 - jr) * 4 >= THREADS ? kRowSmall : 4;
+    const int j = jr + (int)threadIdx.x;
+    if (j < a1) {
+      const int k = ld_stream(acol + j);
+      const double a = aval ? ldv_stream(aval + j) : 0.0;
+      const int s0 = __ldg(brpt + k), s1 = __ldg(brpt + k + 1);
+      if (s1 - s0 <= small_max) {
+        int e = s0;
+        for (; e + 4 <= s1; e += 4) {
+          const int c0 = __ldg(bcol + e), c1 = __ldg(bcol + e + 1);
+          const int c2 = __ldg(bcol + e + 2), c3 = __ldg(bcol + e + 3);
+          const double b0 = bv(e), b1 = bv(e + 1), b2 = bv(e + 2), b3 = bv(e + 3);
+          f(c0, a, b0);
+          f(c1, a, b1);
+          f(c2, a, b2);
+          f(c3, a, b3);
+        }
+        for (; e < s1; ++e) f(__ldg(bcol + e), a, bv(e));
+      } else {
+        const int big = (s1 - s0 >= THREADS) ? 1 : 0;
+        const int slot = atomicAdd(&rq.ctr[par][big], 1);
+        rq.q[big ? THREADS - 1 - slot : slot] =
+            make_int4(s0, s1, __double2loint(a), __double2hiint(a));
+      }
+    }
+    __syncthreads();
+    // the other counter set was last read before the previous round's closing
+    // barrier and is next written after this round's
+    if (threadIdx.x == 0) rq.ctr[par ^ 1][0] = rq.ctr[par ^ 1][1] = rq.ctr[par ^ 1][2] = 0;
+    const int nm = rq.ctr[par][0], nb = rq.ctr[par][1];
+    for (;;) {
+      int i = 0;
+      if (lane == 0) i = atomicAdd(&rq.ctr[par][2], 1);
+      i = __shfl_sync(0xffffffffu, i, 0);
+      if (i >= nm) break;
+      const int4 v = rq.q[i];
+      strided(v.x + lane, v.y, __hiloint2double(v.w, v.z), std::integral_constant<int, 32>());
+    }
+    unsigned pos = 0;  // products of the long rows before row i, mod 2^32
+    for (int i = 0; i < nb; ++i) {
+      const int4 v = rq.q[THREADS - 1 - i];
+      const int first = (int)((threadIdx.x - pos) & (unsigned)(THREADS - 1));
+      strided(v.x + first, v.y, __hiloint2double(v.w, v.z),
+              std::integral_constant<int, THREADS>());
+      pos += (unsigned)(v.y - v.x);
+    }
+    __syncthreads();
+  }
+  // counters of the last round (the other set was cleared during it); the
+  // caller's barrier before the next call orders this
+  if (a1 > a0 && threadIdx.x == 0)
+    rq.ctr[par ^ 1][0] = rq.ctr[par ^ 1][1] = rq.ctr[par ^ 1][2] = 0;
 }
 
 // Intermediate products of one A row and the range of columns they can

@@ -86,6 +86,7 @@ struct ProdInfo {
   int max_brows = 0;
   long long brows = 0;  // rows of every product's B
   bool bdel = false;    // a table whose products have room for their B row shifts
+  double mean_b = 0;    // mean length of the B rows read (once the products are counted)
 };
 
 // Inclusive row limits of the symbolic and numeric bins (the last bin of each

@@ -281,7 +281,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *red, int *tot) {
   return r;
 }
 
-template <int LOG2T, typename VT, bool MULTI>
+template <int LOG2T, typename VT, bool MULTI, bool LONG>
 __global__ void __launch_bounds__(kNumBlockThreads, num_block_minb(LOG2T))
     k_num_block(const ProdTable<VT> src, const int *__restrict__ crpt, int *__restrict__ ccol,
                 double *__restrict__ cval, const int *__restrict__ rows, int count,
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(kNumBlockThreads, num_block_minb(LOG2T))
   int *cnt = bkeys + H;
   __shared__ int red[kNumBlockThreads / 32];
   __shared__ int s_mn, s_mx, s_slot;
-  __shared__ RowQueue<kNumBlockThreads> rq;
+  __shared__ RowQueueOf<kNumBlockThreads, LONG> rq;
   row_queue_init(rq);
   const int lane = threadIdx.x & 31;
   int rows_done = 0;
@@ -454,7 +454,7 @@ __device__ __forceinline__ void red_add_global_keep(double *p, double v, unsigne
                : "memory");
 }
 
-template <typename VT, int MINB, bool MULTI>
+template <typename VT, int MINB, bool MULTI, bool LONG>
 __global__ void __launch_bounds__(kRankThreads, MINB)
     k_num_rank(const ProdTable<VT> src, int b_sorted, int pl_max, const int *__restrict__ crpt,
                int *__restrict__ ccol, double *__restrict__ cval,
@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(kRankThreads, MINB)
   double *vals = reinterpret_cast<double *>(pre + max_words);  // max_words*2: multiple of 8
   __shared__ int base[kRankThreads / 32];
   __shared__ int s_total, s_slot;
-  __shared__ RowQueue<kRankThreads> rq;
+  __shared__ RowQueueOf<kRankThreads, LONG> rq;
   __shared__ SpanScratch<kRankThreads> sc;
   row_queue_init(rq);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -599,8 +599,11 @@ static cudaError_t run_num_rank(const ProdTable<VT> &t, const ProdInfo &info, bo
   const int pl = rank_per_log2((int)std::min<long long>(info.max_ncols, kRankMaxCols));
   const int smem = rank_smem(pl);
   const bool multi = t.prod_of_row != nullptr;
-  auto kern = rank_minb(pl) == 1 ? (multi ? k_num_rank<VT, 1, true> : k_num_rank<VT, 1, false>)
-                                 : (multi ? k_num_rank<VT, 2, true> : k_num_rank<VT, 2, false>);
+  const bool one = rank_minb(pl) == 1;
+#define NSPB_NR(MINB, LONG) (multi ? k_num_rank<VT, MINB, true, LONG> : k_num_rank<VT, MINB, false, LONG>)
+  auto kern = info.mean_b > kLongMean ? (one ? NSPB_NR(1, true) : NSPB_NR(2, true))
+                          : (one ? NSPB_NR(1, false) : NSPB_NR(2, false));
+#undef NSPB_NR
   const int grid = persistent_grid((const void *)kern, kRankThreads, smem, count, 1);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
   kern<<<grid, kRankThreads, smem, s>>>(t, b_sorted ? 1 : 0, pl, crpt, ccol, cval, rows, count,
@@ -642,12 +645,14 @@ static cudaError_t num_group_bin(int bin, const ProdTable<VT> &t, const int *crp
 }
 
 template <int LOG2T, typename VT>
-static cudaError_t run_num_block(const ProdTable<VT> &t, const int *crpt, int *ccol,
+static cudaError_t run_num_block(const ProdTable<VT> &t, bool long_b, const int *crpt, int *ccol,
                                  double *cval, const int *rows, int count, int *err, int *redo,
                                  int *ticket, const int *dcount, cudaStream_t s) {
   constexpr int T = 1 << LOG2T;
   const int smem = T * 12 + (T / 2) * 12 + (T / 2) * 4;
-  auto kern = t.prod_of_row ? k_num_block<LOG2T, VT, true> : k_num_block<LOG2T, VT, false>;
+  const bool multi = t.prod_of_row != nullptr;
+  auto kern = long_b ? (multi ? k_num_block<LOG2T, VT, true, true> : k_num_block<LOG2T, VT, false, true>)
+                     : (multi ? k_num_block<LOG2T, VT, true, false> : k_num_block<LOG2T, VT, false, false>);
   const int grid = persistent_grid((const void *)kern, kNumBlockThreads, smem, count, 1);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
   kern<<<grid, kNumBlockThreads, smem, s>>>(t, crpt, ccol, cval, rows, count, err, redo, ticket,
@@ -681,14 +686,14 @@ static cudaError_t numeric_bin_t(int bin, int lanes, bool owned, bool b_sorted,
                             ticket, s);
   switch (bin) {
     case kNumGroupBins:
-      return run_num_block<11, VT>(t, crpt, ccol, cval, rows, count, err, redo, ticket, dcount,
-                                   s);
+      return run_num_block<11, VT>(t, info.mean_b > kLongMeanBlock, crpt, ccol, cval, rows, count, err, redo, ticket,
+                                   dcount, s);
     case kNumGroupBins + 1:
-      return run_num_block<12, VT>(t, crpt, ccol, cval, rows, count, err, redo, ticket, dcount,
-                                   s);
+      return run_num_block<12, VT>(t, info.mean_b > kLongMeanBlock, crpt, ccol, cval, rows, count, err, redo, ticket,
+                                   dcount, s);
     default:
-      return run_num_block<13, VT>(t, crpt, ccol, cval, rows, count, err, redo, ticket, dcount,
-                                   s);
+      return run_num_block<13, VT>(t, info.mean_b > kLongMeanBlock, crpt, ccol, cval, rows, count, err, redo, ticket,
+                                   dcount, s);
   }
 }
 

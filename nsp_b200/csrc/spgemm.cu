@@ -411,6 +411,7 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
   // them: a block-diagonal batch mixes products whose B rows differ
   if (!(opts.group_lanes == 8 || opts.group_lanes == 16 || opts.group_lanes == 32) && a_nnz > 0)
     lanes = pick_lanes((double)intprod / (double)a_nnz, (double)a_nnz / (double)n, n);
+  if (a_nnz > 0) info.mean_b = (double)intprod / (double)a_nnz;
   int nonempty = 0, binned = 0;
   BinOffsets off = offsets_of(todo, kSymBins, &nonempty, &binned);
   const bool direct = nonempty == 1 && binned == n;
@@ -675,7 +676,9 @@ int Call::prepare_numeric(const int *crpt) {
   if ((st = fetch_counters())) return st;
   b_sorted = opts.assume_sorted || !(h.flags & B_UNSORTED);
   num_counts_ready = true;
-  intprod = (int64_t)h.total_ip;  // 0 where the row walk was skipped
+  intprod = (int64_t)h.total_ip;  // 0 where the row walk was skipped: B's mean row then
+  if (intprod > 0 && a_nnz > 0) info.mean_b = (double)intprod / (double)a_nnz;
+  else if (info.brows > 0) info.mean_b = (double)b_nnz / (double)info.brows;
   if ((st = build_programs()) == NSPB_ERR_ALLOC) drop_runs();
   else if (st) return st;
   if (use_runs) {

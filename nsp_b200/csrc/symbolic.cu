@@ -487,14 +487,14 @@ __host__ __device__ constexpr int sym_wide_minb(int smem) {
   return smem <= kWideTwoBlockSmem ? 2 : 1;
 }
 
-template <bool MULTI, int MINB>
+template <bool MULTI, int MINB, bool LONG>
 __global__ void __launch_bounds__(kWideThreads, MINB)
     k_sym_wide(const ProdTable<void> src, int b_sorted, const int *__restrict__ rows, int count,
                int *__restrict__ row_nz, int *__restrict__ err, int *__restrict__ ticket) {
   extern __shared__ __align__(16) unsigned bm[];
   __shared__ int red[kWideThreads / 32];
   __shared__ int s_slot;
-  __shared__ RowQueue<kWideThreads> rq;
+  __shared__ RowQueueOf<kWideThreads, LONG> rq;
   __shared__ SpanScratch<kWideThreads> sc;
   row_queue_init(rq);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -637,8 +637,11 @@ cudaError_t launch_symbolic_bin(int bin, int lanes, bool b_sorted, const ProdTab
   // the full 128 KB, which it only uses when B has more columns than a window
   const int smem = (int)std::min<long long>(kLongWords, ((long long)info.max_ncols + 31) >> 5) * 4;
   const bool multi = t.prod_of_row != nullptr;
-  auto kern = sym_wide_minb(smem) == 2 ? (multi ? k_sym_wide<true, 2> : k_sym_wide<false, 2>)
-                                       : (multi ? k_sym_wide<true, 1> : k_sym_wide<false, 1>);
+  const bool two = sym_wide_minb(smem) == 2;
+#define NSPB_SW(MINB, LONG) (multi ? k_sym_wide<true, MINB, LONG> : k_sym_wide<false, MINB, LONG>)
+  auto kern = info.mean_b > kLongMean ? (two ? NSPB_SW(2, true) : NSPB_SW(1, true))
+                          : (two ? NSPB_SW(2, false) : NSPB_SW(1, false));
+#undef NSPB_SW
   const int grid = persistent_grid((const void *)kern, kWideThreads, smem, count, 1);
   if (grid <= 0) return cudaErrorInvalidConfiguration;
   kern<<<grid, kWideThreads, smem, s>>>(t, b_sorted ? 1 : 0, rows, count, row_nz, err, ticket);
