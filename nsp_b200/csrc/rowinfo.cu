@@ -87,9 +87,10 @@ constexpr int kRowinfoLong = 1024;
 // than kInfoSerial entries on average and for fewer than kGroupInfoRows rows.
 // The tiles of k_rowinfo keep few threads busy there (products of every row,
 // this kernel and the tiles: 50,000 rows of 700 entries 132 and 289 us, 2000 of
-// 300 39 and 52, 8000 of 27 39 and 45; 33,000 of 27 46 and 40 the other way).
+// 300 39 and 52; the kernels alone, 10,000 of 27 7 and 12; 33,000 of 27 46 and
+// 40 the other way).
 constexpr int kInfoSerial = 64;
-constexpr int kGroupInfoRows = 10000;
+constexpr int kGroupInfoRows = 16000;
 template <int GA, bool MULTI>
 __global__ void __launch_bounds__(256)
     k_rowinfo_group(const ProdTable<void> src, int n, const BinLimits lim,

@@ -32,7 +32,7 @@ LENGTHS = {
 
 
 @pytest.mark.parametrize("kind", LENGTHS)
-@pytest.mark.parametrize("n", [1, 255, 9999, 10000, 10257])
+@pytest.mark.parametrize("n", [1, 255, 15999, 16000, 16257])
 def test_row_products(cuda, n, kind):
     rng = np.random.default_rng(n)
     k = 6007
@@ -46,7 +46,7 @@ def test_row_products(cuda, n, kind):
     assert total == want.sum()
 
 
-@pytest.mark.parametrize("n", [2000, 12000])
+@pytest.mark.parametrize("n", [2000, 17000])
 def test_order_is_checked_on_the_way(cuda, n):
     rng = np.random.default_rng(3)
     lens = rng.choice([0, 2, 63, 64, 65, 100], n, p=[.2, .5, .1, .05, .05, .1])
@@ -67,7 +67,7 @@ def test_order_is_checked_on_the_way(cuda, n):
 def test_tiles_across_products(cuda):
     rng = np.random.default_rng(4)
     pairs = []
-    for n in (4097, 5001, 33, 4500):
+    for n in (4097, 5001, 33, 7500):
         k = 700
         A = csr(rng.choice([0, 1, 5, 64, 65, 130], n, p=[.2, .4, .3, .04, .03, .03]), k, rng)
         pairs.append((A, csr(rng.integers(0, 6, k), 5000, rng)))
