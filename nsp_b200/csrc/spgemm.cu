@@ -456,8 +456,12 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
     if ((e = order_block_bins(row_nz, 0, todo, kSymGroupBins, kSymBins, off)) != cudaSuccess)
       return cuda_fail(e);
   }
-  // flat product lists unless the B rows fill the lanes of a row group
+  // flat product lists unless the B rows fill the lanes of a row group; rows of
+  // at most 48 products, which leave most of a warp of the flat kernel idle,
+  // also stay with row groups of 8 lanes (5-point 1000^2 renumbered 165 us
+  // against 255; 300,000 rows of 25 products 58 and 86, of 4 products 26 and 69)
   const bool flat = family() == 0 && (double)intprod < 0.75 * (double)lanes * (double)a_nnz;
+  const int flat_from = lanes == 8 ? 2 : 0;
   for (int b = 0; b < kSymBins; ++b) {
     const int c = todo[b];
     if (c <= 0) continue;
@@ -472,7 +476,7 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
       m.chunk = template_run();
       m.bshift = bshift;
       e = launch_symbolic_map(b, lanes, structure_of(t64), rows, c, row_nz, &ctr->err, m, s);
-    } else if (b < kSymGroupBins && flat) {
+    } else if (b < kSymGroupBins && flat && b >= flat_from) {
       e = launch_symbolic_flat(b, structure_of(t64), rows, c, row_nz, &ctr->err, s);
     } else {
       e = launch_symbolic_bin(b, lanes, b_sorted, structure_of(t64), info, rows, c, row_nz,
@@ -563,6 +567,7 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
   // rows that the flat kernels leave, of the row-group bins and of the others
   // (row_nz is free by now), and how many
   const bool flat = use_flat();
+  const bool few = info.mean_b * (double)a_nnz <= 12.0 * (double)n;
   int *over[2] = {row_nz, row_nz + off.v[kNumGroupBins]};
   int *n_over[2] = {&ctr->ticket[26], &ctr->ticket[27]};
   int flat_rows[2] = {0, 0};
@@ -598,7 +603,10 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
       ++launches;
       continue;
     }
-    if (b < kNumLong && flat) {
+    // rows of at most 16 entries and few products on average: row groups of 8
+    // lanes (300,000 rows of 4 products 93 us, from flat lists 161; 1 M of 9 380
+    // and 526; the short rows of a power-law 300,000^2 of mean 6 170 and 126)
+    if (b < kNumLong && flat && !(b == 0 && lanes == 8 && few)) {
       const int k = b >= kNumGroupBins;
       e = comp ? launch_numeric_comp_flat(b, b_sorted, t32, crpt, ccol, cval, rows, c, nmax,
                                           &ctr->redo_count, &ctr->max_comp_deg, over[k], n_over[k],
