@@ -564,13 +564,25 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
       launches += 2;
     }
   }
-  // rows that the flat kernels leave, of the row-group bins and of the others
-  // (row_nz is free by now), and how many
+  // Rows with more products than their flat list holds go to the hash kernel
+  // of their own bin (of bin 3 for the smaller ones): with one kernel for all
+  // rows of up to 512 entries and one for the others, 10,000 rows of 996 entries
+  // and 1296 products took 608 us there, 298 in their own. Where products exceed
+  // the entries by 5% at most there can be few such rows, and two launches do.
+  // Bin b's are listed from off.v[b] on (row_nz is free by now).
+  const bool apart = intprod <= 0 || (double)intprod > 1.05 * (double)h.total_nnz;
+  constexpr int kFlatFirst = 3;
+  auto over_bin = [&](int b) {
+    if (!apart) return b < kNumGroupBins ? kNumGroupBins - 1 : kNumLong - 1;
+    return std::max(b, kFlatFirst);
+  };
+  auto over_at = [&](int bin) {
+    if (!apart) return off.v[bin < kNumGroupBins ? 0 : kNumGroupBins];
+    return off.v[bin == kFlatFirst ? 0 : bin];
+  };
   const bool flat = use_flat();
   const bool few = info.mean_b * (double)a_nnz <= 12.0 * (double)n;
-  int *over[2] = {row_nz, row_nz + off.v[kNumGroupBins]};
-  int *n_over[2] = {&ctr->ticket[26], &ctr->ticket[27]};
-  int flat_rows[2] = {0, 0};
+  int flat_rows[kNumLong] = {};
   for (int b = 0; b < kNumBins; ++b) {
     const int c = todo[b];
     if (c <= 0) continue;
@@ -607,26 +619,26 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
     // lanes (300,000 rows of 4 products 93 us, from flat lists 161; 1 M of 9 380
     // and 526; the short rows of a power-law 300,000^2 of mean 6 170 and 126)
     if (b < kNumLong && flat && !(b == 0 && lanes == 8 && few)) {
-      const int k = b >= kNumGroupBins;
+      const int o = over_bin(b);
+      int *over = row_nz + over_at(o);
       e = comp ? launch_numeric_comp_flat(b, b_sorted, t32, crpt, ccol, cval, rows, c, nmax,
-                                          &ctr->redo_count, &ctr->max_comp_deg, over[k], n_over[k],
-                                          &ctr->err, s)
-               : launch_numeric_flat(b, t64, crpt, ccol, cval, rows, c, over[k], n_over[k],
+                                          &ctr->redo_count, &ctr->max_comp_deg, over,
+                                          &ctr->over[o], &ctr->err, s)
+               : launch_numeric_flat(b, t64, crpt, ccol, cval, rows, c, over, &ctr->over[o],
                                      &ctr->err, s);
       if (e != cudaSuccess) return cuda_fail(e);
       ++launches;
-      flat_rows[k] += c;
+      flat_rows[o] += c;
       continue;
     }
     if ((e = hash_bin(b, lanes, rows, c, ticket, tshift, nullptr)) != cudaSuccess)
       return cuda_fail(e);
     ++launches;
   }
-  for (int k = 0; k < 2; ++k) {
-    if (flat_rows[k] == 0) continue;
-    const int b = k ? kNumLong - 1 : kNumGroupBins - 1;
-    if ((e = hash_bin(b, 32, over[k], flat_rows[k], &ctr->ticket[16 + b], 0, n_over[k])) !=
-        cudaSuccess)
+  for (int b = 0; b < kNumLong; ++b) {
+    if (flat_rows[b] == 0) continue;
+    if ((e = hash_bin(b, apart ? lanes : 32, row_nz + over_at(b), flat_rows[b],
+                      &ctr->ticket[16 + b], 0, &ctr->over[b])) != cudaSuccess)
       return cuda_fail(e);
     ++launches;
   }

@@ -30,14 +30,18 @@ struct DevCounters {
   int pad;
   int ticket[32];    // row tickets of the block-per-row launches (symbolic
                      // bin b at b, numeric bin b at 16 + b; the runs at 30,
-                     // 31, the bunches at 28, 29; at 26, 27 the rows that
-                     // k_num_flat left to the hash kernels)
+                     // 31, the bunches at 28, 29)
+  int over[12];      // rows that k_num_flat left to the hash kernel of each bin
   // from here on only with row runs (Call::counter_bytes)
   int lag_count[4];  // B rows with a column shift at lag 1, 2, 3
   int sym_sub[16];   // rows of each symbolic bin that belong to a run
   int num_sub[16];   // rows of each numeric bin that do
   RunHead run;
 };
+
+// Part of the scratch that nspb_spgemm_noalloc serves without allocating: a
+// whole number of 256 bytes, so that up to here it costs no rows.
+static_assert(offsetof(DevCounters, lag_count) <= 512, "two units of 256 bytes");
 
 struct HostStage {
   DevCounters c;
