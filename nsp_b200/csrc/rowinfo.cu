@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256)
 // operands the threads of a warp then gather neighbouring entries of B's row
 // pointer; a group of lanes a row waited for pointer, columns and gather in
 // turn (370 us on the 27-point 128^3 stencil, 150 us on the power-law 1M
-// matrix). Rows of more than kInfoSerial entries are left to whole warps,
+// matrix). Rows of more than kInfoSerial entries are left to the whole warp,
 // those of more than kRowinfoLong to k_rowinfo_long.
 
 template <bool MULTI>
@@ -189,9 +189,6 @@ __global__ void __launch_bounds__(kTileThreads)
   __shared__ unsigned long long s_total;
   __shared__ int cols[kTileWords];
   __shared__ int rp[kTileThreads + kMaxLag + 1];  // row starts from three rows before the tile
-  __shared__ short s_far[kTileThreads];           // rows left to a warp
-  __shared__ long long s_sum[kTileThreads];       // and their products
-  __shared__ int s_nfar;
   if (threadIdx.x < kSymBins) hist[threadIdx.x] = 0;
   if (threadIdx.x == 0) s_total = 0ull;
   __syncthreads();
@@ -308,41 +305,29 @@ __global__ void __launch_bounds__(kTileThreads)
         }
       }
       if (flags) bad |= wrong;
-      // longer rows, a warp a row, all warps sharing the tile's (each warp left
-      // to its own 32 rows: 60,000 rows of 70 entries 90 us, 45 now)
-      const bool far = na > kInfoSerial && !code && !listed;
-      if (__syncthreads_or(far)) {
-        if (threadIdx.x == 0) s_nfar = 0;
-        __syncthreads();
-        if (far) s_far[atomicAdd(&s_nfar, 1)] = (short)q;
-        __syncthreads();
-        for (int i = threadIdx.x >> 5; i < s_nfar; i += kTileThreads / 32) {
-          const int w = s_far[i];
-          int b0, b1;
-          Operands<void> ow;
-          if (MULTI && split) {
-            const int lw = prod_row<MULTI>(src, r0 + w, ow);
-            b0 = __ldg(ow.arpt + lw);
-            b1 = __ldg(ow.arpt + lw + 1);
-          } else {
-            ow = o;
-            b0 = rp[w + kMaxLag];
-            b1 = rp[w + kMaxLag + 1];
-          }
-          auto at = [&](int j) { return MULTI && split ? __ldg(ow.acol + j) : col(j); };
-          long long sum = 0;
-#pragma unroll 4
-          for (int j = b0 + lane; j < b1; j += 32) {
-            const int k = at(j);
-            sum += __ldg(ow.brpt + k + 1) - __ldg(ow.brpt + k);
-            if (flags) bad |= j > b0 && k <= at(j - 1);
-          }
-#pragma unroll
-          for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-          if (lane == 0) s_sum[w] = sum;
+      // longer rows, a warp a row
+      unsigned todo = __ballot_sync(0xffffffffu, na > kInfoSerial && !code && !listed);
+      while (todo) {
+        const int w = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        const int b0 = __shfl_sync(0xffffffffu, a0, w), b1 = __shfl_sync(0xffffffffu, a1, w);
+        const int *acol = o.acol, *brpt = o.brpt;
+        if (MULTI && split) {
+          acol = reinterpret_cast<const int *>(
+              __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(acol), w));
+          brpt = reinterpret_cast<const int *>(
+              __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(brpt), w));
         }
-        __syncthreads();
-        if (far) ip = s_sum[q];
+        auto at = [&](int j) { return MULTI && split ? __ldg(acol + j) : col(j); };
+        long long sum = 0;
+        for (int j = b0 + lane; j < b1; j += 32) {
+          const int k = at(j);
+          sum += __ldg(brpt + k + 1) - __ldg(brpt + k);
+          if (flags) bad |= j > b0 && k <= at(j - 1);
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (lane == w) ip = sum;
       }
       if (q >= nr) return;
       if (listed) {
