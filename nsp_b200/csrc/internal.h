@@ -148,30 +148,34 @@ struct RowRun {
   int place;  // among the runs of its pattern
 };
 inline long long run_capacity(long long n) { return n / kRunMin + 1; }
-// The patterns of the runs: a table of representatives (run index + 1, 0:
-// free), the program of each slot and the representative run of each program.
+// The patterns of the runs: a table of representatives (hash of the pattern << 32
+// | run index + 1, 0: free), the program of each slot and the representative run
+// of each program. Only a representative of the same hash is compared with.
 constexpr int kRunSlots = 4096;
 struct RunHead {
   int nfound;    // runs found
   int nprog;     // patterns among them
   int nruns[2];  // runs kept: of few, of many products a row
   int nbunch;    // bunches: patterns shared by rows that are in no run
-  int pad[3];
+  int bnew;      // leftover rows that met no earlier row's pattern
+  int pad[2];    // a multiple of 8 bytes: the tables follow
 };
 struct RunTable {
   RunHead *head = nullptr;
-  int *rep = nullptr, *prog_of = nullptr, *run_of = nullptr;  // kRunSlots each; rep zeroed
+  unsigned long long *rep = nullptr;  // kRunSlots, zeroed; the others kRunSlots each
+  int *prog_of = nullptr, *run_of = nullptr;
   // runs of each slot (zeroed); by program: slot | large << 16, first run in the list
   int *count = nullptr, *slot_of = nullptr, *first = nullptr;
-  // bunches: representative row + 1 and rows of each slot (zeroed), where a
-  // slot's rows are listed (-1: not a bunch), then by bunch: its first row,
-  // rows and place in the list
-  int *brep = nullptr, *bcount = nullptr, *bslot = nullptr;
+  // bunches: representative (hash << 32 | row + 1) and rows of each slot (both
+  // zeroed), where a slot's rows are listed (-1: its rows make no bunch), then
+  // by bunch: its first row, rows and place in the list
+  unsigned long long *brep = nullptr;
+  int *bcount = nullptr, *bslot = nullptr;
   int *brow = nullptr, *brows = nullptr, *bplace = nullptr;
   // tiles of few and of many products a row before each bunch (kRunSlots + 64 each)
   int *btiles[2] = {nullptr, nullptr};
 };
-constexpr int kRunTableZeroed = 4, kRunTableRest = 10;  // tables of kRunSlots ints (+ 64)
+constexpr int kRunTableZeroed = 6, kRunTableRest = 10;  // tables of kRunSlots ints (+ 64)
 
 // fp32 input modes (compensated pairs, or fp64 accumulation of exact products).
 inline bool fp32_inputs(int precision) {

@@ -284,6 +284,11 @@ __device__ __forceinline__ unsigned run_mix(unsigned a, unsigned b) {
   return a ^ (a >> 16);
 }
 
+// An entry of a table of representatives.
+__device__ __forceinline__ unsigned long long run_entry(unsigned hash, int index) {
+  return (unsigned long long)hash << 32 | (unsigned)(index + 1);
+}
+
 // Patterns of the runs: a warp a run hashes everything that its program
 // depends on and looks for a run with the same pattern in a table of
 // representatives; a run that finds one is compared with it, value by value.
@@ -343,10 +348,13 @@ __global__ void __launch_bounds__(256)
     int slot = -1;
     for (int tries = 0; tries < 16 && slot < 0; ++tries) {
       const int at = (int)((h + (unsigned)tries) & (kRunSlots - 1));
-      int rep = 0;
-      if (lane == 0) rep = atomicCAS(rt.rep + at, 0, q + 1);
-      rep = __shfl_sync(0xffffffffu, rep, 0);
-      if (rep == 0) {  // the first of its pattern
+      unsigned long long entry = 0;
+      if (lane == 0) {
+        entry = *(volatile unsigned long long *)(rt.rep + at);
+        if (entry == 0) entry = atomicCAS(rt.rep + at, 0ull, run_entry(h, q));
+      }
+      entry = __shfl_sync(0xffffffffu, entry, 0);
+      if (entry == 0) {  // the first of its pattern
         slot = at;
         if (lane == 0) {
           const int p = atomicAdd(&rt.head->nprog, 1);
@@ -357,6 +365,8 @@ __global__ void __launch_bounds__(256)
         break;
       }
       // the same pattern as the representative's?
+      if ((unsigned)(entry >> 32) != h) continue;
+      const int rep = (int)(unsigned)entry;
       const RowRun other{found[rep - 1].row0, found[rep - 1].meta, 0, 0};
       if ((other.meta >> 2 & 3) != sigma) continue;
       Operands<void> o2;
@@ -438,19 +448,28 @@ cudaError_t launch_run_find(const ProdTable<void> &t, unsigned char *codes, int 
 // computed by the same programs, each row's B values staged on their own. On
 // the 27-point 128^3 stencil the 65,536 rows at the ends of its lines took 297
 // us in k_sym_map and 305 us in k_num_map, a fifth of the product.
+//
+// Rows without structure all differ: hashing 1.6 M of them on a 7-point grid
+// took 1.6 ms of 7.5, and 4096 programs for one row each 0.9 ms more on a
+// 27-point one. The search therefore ends after kBunchNew rows that met no
+// earlier row's pattern (the grids and their aggregation products have 27 to
+// 730 patterns).
+constexpr int kBunchNew = 2048;
 constexpr int kBunchBits = 19;  // place of a row in its slot; slots take the bits above
 static_assert(kRunSlots <= 1 << (31 - kBunchBits), "slot and place in one int");
 
 template <bool MULTI>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, MULTI ? 5 : 8)
     k_bunch_key(const ProdTable<void> src, const unsigned char *__restrict__ member, int n,
                 const int *__restrict__ row_nz, const RunTable rt, int *__restrict__ slot_of) {
   const int lane = threadIdx.x & 31;
   const int warps = gridDim.x * 8;
+  int seen = 0;  // of the last eight rows: looked at, and << 8 those that met no pattern; -1: no more
   for (int base = ((blockIdx.x * 256 + threadIdx.x) >> 5) * 32; base < n; base += warps * 32) {
     const int mine = base + lane;
     int my_slot = -1;
-    unsigned todo = __ballot_sync(0xffffffffu, mine < n && !member[mine] && row_nz[mine] > 0);
+    unsigned todo =
+        __ballot_sync(0xffffffffu, seen >= 0 && mine < n && !member[mine] && row_nz[mine] > 0);
     while (todo) {
       const int w = __ffs(todo) - 1;
       todo &= todo - 1u;
@@ -501,16 +520,19 @@ __global__ void __launch_bounds__(256)
       int slot = -1;
       for (int tries = 0; tries < 16 && slot < 0; ++tries) {
         const int at = (int)((h + (unsigned)tries) & (kRunSlots - 1));
-        int rep = 0;
+        unsigned long long entry = 0;
         if (lane == 0) {
-          rep = *(volatile int *)(rt.brep + at);
-          if (rep == 0) rep = atomicCAS(rt.brep + at, 0, row + 1);
+          entry = *(volatile unsigned long long *)(rt.brep + at);
+          if (entry == 0) entry = atomicCAS(rt.brep + at, 0ull, run_entry(h, row));
         }
-        rep = __shfl_sync(0xffffffffu, rep, 0);
-        if (rep == 0) {
+        entry = __shfl_sync(0xffffffffu, entry, 0);
+        if (entry == 0) {
           slot = at;
+          seen += 0x100;
           break;
         }
+        if ((unsigned)(entry >> 32) != h) continue;
+        const int rep = (int)(unsigned)entry;
         Operands<void> o2;
         const int lr2 = prod_row<MULTI>(src, rep - 1, o2);
         if constexpr (MULTI)
@@ -545,6 +567,17 @@ __global__ void __launch_bounds__(256)
         if (!diff) slot = at;
       }
       int place = 0;
+      seen += slot < 0 ? 0x101 : 1;
+      if ((seen & 0xff) == 8) {
+        if (seen >= 0x100) {
+          int before = 0;
+          if (lane == 0) before = atomicAdd(&rt.head->bnew, seen >> 8);
+          seen = __shfl_sync(0xffffffffu, before, 0) >= kBunchNew ? -1 : 0;
+          if (seen < 0) todo = 0;
+        } else {
+          seen = 0;
+        }
+      }
       if (slot >= 0) {
         if (lane == 0) place = atomicAdd(rt.bcount + slot, 1);
         place = __shfl_sync(0xffffffffu, place, 0);
@@ -555,15 +588,34 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Used slots become bunches, in slot order; one block, kRunSlots / 1024 slots a thread.
+// Used slots become bunches, in slot order; one block, kRunSlots / 1024 slots a
+// thread. Where there are more than kBunchAll patterns, those of fewer than
+// kBunchMin rows are left to the other kernels: a program takes as long as those
+// need for about 24 rows (0.2 us).
+constexpr int kBunchAll = 1024, kBunchMin = 24;
+
 __global__ void __launch_bounds__(1024) k_bunch_plan(const RunTable rt) {
   constexpr int kPer = kRunSlots / 1024;
   __shared__ int s_rows[32], s_num[32];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  int c[kPer], rows = 0, num = 0;
+  int c[kPer], used = 0;
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
     c[i] = min(rt.bcount[t * kPer + i], 1 << kBunchBits);
+    used += c[i] > 0;
+  }
+  used = __reduce_add_sync(0xffffffffu, used);
+  if (lane == 0) s_num[warp] = used;
+  __syncthreads();
+  const bool many = __reduce_add_sync(0xffffffffu, s_num[lane]) > kBunchAll;
+  __syncthreads();  // s_num
+  int rows = 0, num = 0;
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    if (many && c[i] < kBunchMin) {
+      rt.bslot[t * kPer + i] = -1;
+      c[i] = 0;
+    }
     rows += c[i];
     num += c[i] > 0;
   }
@@ -592,7 +644,7 @@ __global__ void __launch_bounds__(1024) k_bunch_plan(const RunTable rt) {
     if (c[i] == 0) continue;
     const int slot = t * kPer + i;
     rt.bslot[slot] = place;
-    rt.brow[b] = rt.brep[slot] - 1;
+    rt.brow[b] = (int)(unsigned)rt.brep[slot] - 1;
     rt.brows[b] = c[i];
     rt.bplace[b] = place;
     place += c[i];
@@ -610,7 +662,9 @@ __global__ void __launch_bounds__(256)
   for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
     const int v = slot_of[i];
     if (v < 0) continue;
-    list[rt.bslot[v >> kBunchBits] + (v & ((1 << kBunchBits) - 1))] = i;
+    const int first = rt.bslot[v >> kBunchBits];
+    if (first < 0) continue;
+    list[first + (v & ((1 << kBunchBits) - 1))] = i;
     member[i] = 1;
     const int ub = row_nz[i];
     if (ub > 0) atomicAdd(&hist[sym_bin(ub, lim)], 1);

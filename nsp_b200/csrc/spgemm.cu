@@ -189,10 +189,10 @@ int Call::alloc_scratch() {
   tile_state = reinterpret_cast<unsigned long long *>(ws + off_tiles);
   if (allow_runs) {
     rtab.head = &ctr->run;
-    rtab.rep = reinterpret_cast<int *>(ctr + 1);
+    rtab.rep = reinterpret_cast<unsigned long long *>(ctr + 1);
     rtab.prog_of = reinterpret_cast<int *>(ws + off_slots);
     rtab.brep = rtab.rep + kRunSlots;
-    rtab.bcount = rtab.brep + kRunSlots;
+    rtab.bcount = reinterpret_cast<int *>(rtab.brep + kRunSlots);
     rtab.count = rtab.bcount + kRunSlots;
     int *rest = rtab.prog_of;
     for (int **p : {&rtab.run_of, &rtab.slot_of, &rtab.first, &rtab.bslot, &rtab.brow, &rtab.brows, &rtab.bplace, &rtab.btiles[0],
