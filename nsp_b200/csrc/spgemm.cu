@@ -271,13 +271,22 @@ static BinOffsets offsets_of(const int *counts, int nb, int *nonempty, int *tota
 // vs 519, of 60^3 (11 M) 404 vs 262; B's rows of 4.5 and 7: A P of 48^3 (12 M)
 // 341 vs 390, of 40^3 (7.4 M) 310 vs 284, 7-point 64^3 (12.5 M) 286 vs 406,
 // 64 x 50 x 50 (7.6 M) 249 vs 314, 32^3 (1.5 M) 222 vs 170.
+// The symbolic and the numeric step in calls of their own (two_calls) search
+// twice, and need more: 14 million where B's rows are shorter than 8, 26 million
+// up to 16 if A's have at most 64 entries, 32 million otherwise. Both calls, runs against what came before
+// them: A P of 44^3 (9.8 M) 585 vs 460, of 52^3 (16.6 M) 649 vs 672; 7-point
+// 12.5 M 515 vs 497, 17.9 M 605 vs 646; R (A P) of 80^3 873 vs 818, 15-point
+// 26.6 M 539 vs 657; 27-point 31 M 566 vs 523, 43 M 608 vs 686.
 bool Call::runs_wanted() const {
   if (!allow_runs || family() != 0 || (opts.row_kernel & kNoRowTemplates)) return false;
   if (n < 2 * kRunMin || a_nnz > (int64_t)kRunMaxA * n || (table && !info.bdel)) return false;
   if ((opts.row_kernel & 0xff) == 8) return true;
   if (info.brows <= 0) return false;
   const double mean = (double)b_nnz / (double)info.brows;
-  return (double)a_nnz * mean >= (mean < 8.0 ? 8e6 : 24e6);
+  const double least = mean < 8.0 ? (two_calls ? 14e6 : 8e6)
+                       : !two_calls ? 24e6
+                       : mean < 16.0 && a_nnz <= 64LL * n ? 26e6 : 32e6;
+  return (double)a_nnz * mean >= least;
 }
 
 int Call::alloc_runs() {
@@ -672,6 +681,7 @@ bool Call::map_wanted() const {
 // Numeric bins and B order for a two-call numeric step.
 int Call::prepare_numeric(const int *crpt) {
   if (n == 0) return NSPB_OK;
+  two_calls = true;
   int st = alloc_scratch();
   if (st) return st;
   cudaError_t e;
@@ -812,6 +822,7 @@ int nspb_spgemm_symbolic(const nspb_csr_in *A, const nspb_csr_in *B, nspb_csr_ou
   int st = call.init(A, B, opts);
   if (st) return st;
   call.allow_map = false;  // the numeric phase runs in another call
+  call.two_calls = true;
   bool own_rpt = false;
   if (!C->rowptr) {
     if ((st = alloc_out(reinterpret_cast<void **>(&C->rowptr), ((size_t)call.n + 1) * 4))) return st;

@@ -104,6 +104,7 @@ struct Call {
   // counted once a run and computed by k_num_run. allow_runs false: entry
   // points that may not allocate.
   bool allow_runs = true;
+  bool two_calls = false;  // the other phase is another call's
   bool use_runs = false;
   int nruns[2] = {0, 0};       // of few, of many products a row
   char *run_block = nullptr;   // pool block: member flags, runs, B row shifts
