@@ -253,6 +253,14 @@ constexpr double kLongMean = 56.0, kLongMeanBlock = 128.0;
 template <int THREADS, bool LONG>
 using RowQueueOf = std::conditional_t<LONG, RowWarpQueue<THREADS>, RowQueue<THREADS>>;
 
+// B rows of at most this many entries need no list (row_products) in a launch of
+// `rows` rows. The list is ahead from three entries on, and with very few rows,
+// where a block's latency is all there is, from about eight: A rows of 20000 or
+// 200000 entries over B rows of 1, 2, 3, 4 or 6, list and thread a row, 300 rows
+// 846 and 689, 1046 and 971, 1288 and 1366, 1479 and 1629, 2152 and 2598 us, one
+// row 1705 and 1202, 2104 and 1559, 2502 and 1972, 2857 and 2494, 3635 and 3296.
+__device__ __forceinline__ int row_few(int rows) { return rows <= 16 ? 6 : 2; }
+
 // Every product of one A row, spread evenly over a block of THREADS threads
 // whatever the lengths of the B rows it touches (power-law matrices mix rows
 // of one entry with hub rows of 10^4 and more). The A row is taken in rounds
@@ -263,16 +271,17 @@ using RowQueueOf = std::conditional_t<LONG, RowWarpQueue<THREADS>, RowQueue<THRE
 // consecutive products, lane l the product l of the piece, so that every lane
 // works and neighbours read neighbouring B entries. U pieces' loads are in
 // flight at a time in each warp.
+// A round without a B row of more than row_few(rows) entries (rows: of the launch)
+// makes no list: a thread walks the row of its own entry.
 // f(c, a, b) gets the B entry's column, the A value and the B value (values 0
 // when aval / bval are null). Every thread of the block must call this with
-// the same (a0, a1) after a block barrier, and a block barrier must separate
-// two calls.
+// the same (a0, a1) after a block barrier, and a block barrier must follow it.
 template <int THREADS, int U, typename VT, typename F>
 __device__ __forceinline__ void row_products(const int *__restrict__ acol,
                                              const VT *__restrict__ aval,
                                              const int *__restrict__ brpt,
                                              const int *__restrict__ bcol,
-                                             const VT *__restrict__ bval, int a0, int a1,
+                                             const VT *__restrict__ bval, int a0, int a1, int rows,
                                              RowQueue<THREADS> &rq, F &&f) {
   static_assert((THREADS & (THREADS - 1)) == 0 && THREADS <= 1024,
                 "a power of two; the packed scan holds 20 bits of products");
@@ -299,6 +308,7 @@ __device__ __forceinline__ void row_products(const int *__restrict__ acol,
       s0 = __ldg(brpt + k);
       len = __ldg(brpt + k + 1) - s0;
     }
+    const bool list = len > row_few(rows);
     if (len >= THREADS) {
       const int slot = THREADS - 1 - atomicAdd(&rq.big, 1);
       rq.start[slot] = s0;
@@ -315,7 +325,11 @@ __device__ __forceinline__ void row_products(const int *__restrict__ acol,
       if (lane >= o) incl += t;
     }
     if (lane == 31) rq.red[warp] = incl;
-    __syncthreads();
+    if (!__syncthreads_or(list)) {
+#pragma unroll 1
+      for (; len > 0; --len, ++s0) f(__ldg(bcol + s0), a, bv(s0));
+      continue;
+    }
     const unsigned mine = lane < NW ? rq.red[lane] : 0u;
     const unsigned all = __reduce_add_sync(0xffffffffu, mine);
     const unsigned ex = incl - v + __reduce_add_sync(0xffffffffu, lane < warp ? mine : 0u);
@@ -390,7 +404,7 @@ __device__ __forceinline__ void row_products(const int *__restrict__ acol,
                                              const VT *__restrict__ aval,
                                              const int *__restrict__ brpt,
                                              const int *__restrict__ bcol,
-                                             const VT *__restrict__ bval, int a0, int a1,
+                                             const VT *__restrict__ bval, int a0, int a1, int,
                                              RowWarpQueue<THREADS> &rq, F &&f) {
   static_assert((THREADS & (THREADS - 1)) == 0, "THREADS must be a power of two");
   const int lane = threadIdx.x & 31;

@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kNumBlockThreads, num_block_minb(LOG2T))
     const int lr = prod_row<MULTI>(src, row, op);
     const int a0 = op.arpt[lr], a1 = op.arpt[lr + 1];
     int mn = 0x7fffffff, mx = -1;
-    row_products<kNumBlockThreads, 2>(op.acol, op.aval, op.brpt, op.bcol, op.bval, a0, a1, rq,
+    row_products<kNumBlockThreads, 2>(op.acol, op.aval, op.brpt, op.bcol, op.bval, a0, a1, count, rq,
                                    [&](int key, double a, double b) {
       num_insert<LOG2T, false, true>(keys, vals, key, __dmul_rn(a, b), err);
       mn = min(mn, key);
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kRankThreads, MINB)
       const int t0 = threadIdx.x << pl;  // this thread's first word
       // pass 1: distinct columns of the window
       row_products<kRankThreads, (MINB > 1 ? 2 : 4)>(acol, (const VT *)nullptr, brpt, bcol, (const VT *)nullptr, a0,
-                                 a1, rq, [&](int c, double, double) {
+                                 a1, count, rq, [&](int c, double, double) {
         const unsigned d = (unsigned)(c - w0);
         if (d < (unsigned)wn) {
           const unsigned bit = 1u << (d & 31u);
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(kRankThreads, MINB)
           return base[w >> shift] + pre[w] + __popcll(bm64[w] & ((1ull << (d & 63u)) - 1ull));
         };
         if (in_smem) {
-          row_products<kRankThreads, 2>(acol, aval, brpt, bcol, bval, a0, a1, rq,
+          row_products<kRankThreads, 2>(acol, aval, brpt, bcol, bval, a0, a1, count, rq,
                                      [&](int c, double a, double b) {
             const unsigned d = (unsigned)(c - w0);
             if (d < (unsigned)wn) atomicAdd(vals + rank_of(d), __dmul_rn(a, b));
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kRankThreads, MINB)
         } else {
           double *dst = cval + off;
           const unsigned long long pol = l2_evict_last_policy();
-          row_products<kRankThreads, 2>(acol, aval, brpt, bcol, bval, a0, a1, rq,
+          row_products<kRankThreads, 2>(acol, aval, brpt, bcol, bval, a0, a1, count, rq,
                                      [&](int c, double a, double b) {
             const unsigned d = (unsigned)(c - w0);
             if (d < (unsigned)wn) red_add_global_keep(dst + rank_of(d), __dmul_rn(a, b), pol);

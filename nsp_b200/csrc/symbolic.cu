@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(kWideThreads, MINB)
       __syncthreads();
       int nz = 0;
       row_products<kWideThreads, (MINB > 1 ? 2 : 4)>(acol, (const double *)nullptr, brpt, bcol,
-                                 (const double *)nullptr, a0, a1, rq,
+                                 (const double *)nullptr, a0, a1, count, rq,
                                  [&](int c, double, double) {
                                    nz += sym_insert<kWideLog2T, true>(table, c, err);
                                  });
@@ -539,7 +539,7 @@ __global__ void __launch_bounds__(kWideThreads, MINB)
         for (int q = threadIdx.x; q < words; q += kWideThreads) bm[q] = 0u;
         __syncthreads();
         row_products<kWideThreads, (MINB > 1 ? 2 : 4)>(acol, (const double *)nullptr, brpt, bcol,
-                                   (const double *)nullptr, a0, a1, rq,
+                                   (const double *)nullptr, a0, a1, count, rq,
                                    [&](int c, double, double) {
                                      const unsigned d = (unsigned)(c - base);
                                      if (d < (unsigned)wn) {
