@@ -155,6 +155,22 @@ __global__ void __launch_bounds__(FlatCfg<W, K>::TH *FlatCfg<W, K>::ROWS, FlatCf
         col[i] = __ldg(op.bcol + j);
         val[i].set(ft.a[t], __ldg(op.bval + j));
       }
+    // one B row in order is the row of C already
+    bool copy = false;
+    if constexpr (W == 1) {
+      if (ne == 1) {
+        copy = true;
+        int prev = -1;
+#pragma unroll
+        for (int i = 0; i < K; ++i)
+          if (warp_has(i)) {
+            const int left = __shfl_up_sync(0xffffffffu, col[i], 1);
+            copy = copy && (i * C::TH > last || (lane > 0 ? left : prev) < col[i]);
+            prev = __shfl_sync(0xffffffffu, col[i], 31);
+          }
+        copy = __all_sync(0xffffffffu, copy);
+      }
+    }
     int mn = 0x7fffffff, mx = -1;
 #pragma unroll
     for (int i = 0; i < K; ++i)
@@ -183,7 +199,7 @@ __global__ void __launch_bounds__(FlatCfg<W, K>::TH *FlatCfg<W, K>::ROWS, FlatCf
     int at[K];  // bucket | bitmap << 20, then the place
 #pragma unroll
     for (int i = 0; i < K; ++i)
-      if (i * C::TH <= last) {
+      if (!copy && i * C::TH <= last) {
         const int b = bucket_of(col[i], mn, scale, C::WORDS * 32);
         const unsigned bit = 1u << (b & 31);
         int lev = 0;
@@ -195,7 +211,15 @@ __global__ void __launch_bounds__(FlatCfg<W, K>::TH *FlatCfg<W, K>::ROWS, FlatCf
         at[i] = b | lev << 20;
       }
     flat_sync<W>();
-    if (ends[2] == 0) {
+    if (copy) {
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+        if (i * C::TH <= last) {
+          skey[i * C::TH + tid] = col[i];
+          svals[i * C::TH + tid] = val[i];
+        }
+      if (tid == 0) skey[total] = 0x7fffffff;
+    } else if (ends[2] == 0) {
       // products before each word
       uint4 x = reinterpret_cast<const uint4 *>(maps)[tid];
       int4 c = make_int4(__popc(x.x), __popc(x.y), __popc(x.z), __popc(x.w));
