@@ -245,9 +245,17 @@ int scan_tiles(int n);
 cudaError_t launch_scan(const int *row_nz, int n, int *crpt, long long *total,
                         unsigned long long *tile_state, int *tile_ctr, const BinLimits &lim,
                         int *num_counts, int *err, cudaStream_t s);
-// Numeric-bin histogram from an existing row pointer.
+// Numeric-bin histogram from an existing row pointer, and the summed lengths of
+// the B rows that some of A's entries read (samples: 0, or whole blocks of 1024
+// threads of the n rows, 16 at most).
+struct ReadSample {
+  const int *acol = nullptr, *brpt = nullptr;
+  int64_t a_nnz = 0;
+  int samples = 0;
+  int *sum = nullptr;  // zeroed
+};
 cudaError_t launch_num_hist(const int *crpt, int n, const BinLimits &lim, int *num_counts,
-                            cudaStream_t s);
+                            const ReadSample &rs, cudaStream_t s);
 
 // ---- symbolic.cu ----------------------------------------------------------------
 // ticket: a zeroed counter for this launch (block-per-row kernels hand out
@@ -360,8 +368,9 @@ cudaError_t launch_run_find(const ProdTable<void> &t, unsigned char *codes, int 
                             const BinLimits &lim, int *row_nz, RowRun *found,
                             const RunTable &rt, int *sym_sub, cudaStream_t s);
 // The rows left over by the runs, by pattern: rows with one pattern of
-// products form a bunch (a single row too); slot and list (n ints each) are
-// theirs, the rest as in launch_run_find.
+// products form a bunch (a single row too, unless there are many patterns:
+// k_bunch_plan); slot and list (n ints each) are theirs, the rest as in
+// launch_run_find.
 cudaError_t launch_bunch_find(const ProdTable<void> &t, unsigned char *member, int n,
                               const BinLimits &lim, int *row_nz, const RunTable &rt, int *slot,
                               int *list, int *sym_sub, cudaStream_t s);

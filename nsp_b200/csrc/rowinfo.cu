@@ -679,26 +679,40 @@ cudaError_t launch_scan(const int *row_nz, int n, int *crpt, long long *total,
 }
 
 // ---- numeric bins from an existing row pointer ---------------------------------
+// The first rs.samples threads each add the length of the B row that one entry
+// of A reads (at most 65535), the entries spread evenly over A, at a random
+// place within their share so that no pattern of A's rows is met in step.
 __global__ void __launch_bounds__(1024)
     k_num_hist(const int *__restrict__ crpt, int n, const BinLimits lim,
-               int *__restrict__ num_counts) {
+               int *__restrict__ num_counts, const ReadSample rs) {
   __shared__ int hist[kNumBins];
+  __shared__ int s_sum;
   if (threadIdx.x < kNumBins) hist[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_sum = 0;
   __syncthreads();
   const int i = blockIdx.x * 1024 + threadIdx.x;
   if (i < n) {
     const int k = crpt[i + 1] - crpt[i];
     if (k > 0) atomicAdd(&hist[num_bin(k, lim)], 1);
   }
+  if (i < rs.samples) {  // whole blocks
+    const unsigned r = ((unsigned)i * 0x9e3779b1u ^ (unsigned)i >> 7) * 0x85ebca6bu >> 16;
+    const unsigned long long at = ((unsigned long long)i << 16 | r) * (unsigned long long)rs.a_nnz;
+    const int k = __ldg(rs.acol + (at / (unsigned)rs.samples >> 16));
+    const int len = min(__ldg(rs.brpt + k + 1) - __ldg(rs.brpt + k), 0xffff);
+    const int sum = __reduce_add_sync(0xffffffffu, len);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&s_sum, sum);
+  }
   __syncthreads();
   if (threadIdx.x < kNumBins && hist[threadIdx.x])
     atomicAdd(&num_counts[threadIdx.x], hist[threadIdx.x]);
+  if (threadIdx.x == 0 && s_sum) atomicAdd(rs.sum, s_sum);
 }
 
 cudaError_t launch_num_hist(const int *crpt, int n, const BinLimits &lim, int *num_counts,
-                            cudaStream_t s) {
+                            const ReadSample &rs, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  k_num_hist<<<(n + 1023) / 1024, 1024, 0, s>>>(crpt, n, lim, num_counts);
+  k_num_hist<<<(n + 1023) / 1024, 1024, 0, s>>>(crpt, n, lim, num_counts, rs);
   return cudaGetLastError();
 }
 

@@ -406,6 +406,7 @@ int Call::symbolic(int *crpt, int64_t *nnz_out) {
   if ((st = fetch_counters())) return st;
   b_sorted = opts.assume_sorted || !(h.flags & B_UNSORTED);
   intprod = (int64_t)h.total_ip;
+  products = (double)intprod;
   if ((st = build_programs()) == NSPB_ERR_ALLOC) {  // no memory for them: without runs
     drop_runs();
     allow_runs = false;
@@ -579,7 +580,7 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
   // and 1296 products took 608 us there, 298 in their own. Where products exceed
   // the entries by 5% at most there can be few such rows, and two launches do.
   // Bin b's are listed from off.v[b] on (row_nz is free by now).
-  const bool apart = intprod <= 0 || (double)intprod > 1.05 * (double)h.total_nnz;
+  const bool apart = h.total_ip == 0 || products > 1.05 * (double)h.total_nnz;
   constexpr int kFlatFirst = 3;
   auto over_bin = [&](int b) {
     if (!apart) return b < kNumGroupBins ? kNumGroupBins - 1 : kNumLong - 1;
@@ -679,7 +680,7 @@ bool Call::map_wanted() const {
 }
 
 // Numeric bins and B order for a two-call numeric step.
-int Call::prepare_numeric(const int *crpt) {
+int Call::prepare_numeric(const int *crpt, int64_t nnz) {
   if (n == 0) return NSPB_OK;
   two_calls = true;
   int st = alloc_scratch();
@@ -701,14 +702,26 @@ int Call::prepare_numeric(const int *crpt) {
       return cuda_fail(e);
     launches += 3;
   }
-  if ((e = launch_num_hist(crpt, n, lim, ctr->num_counts, s)) != cudaSuccess) return cuda_fail(e);
+  // The products, where they are not counted, are A's entries times B's mean row,
+  // or times the mean row that some of A's entries read where that is clearly
+  // longer (A may read B's long rows above all; the shorter mean would send rows
+  // to lists that they outgrow: 20,000 rows of 10 of B's 400 rows of 60 among
+  // 20,000 of one entry, both calls 414 us, 373 before the lists).
+  const double plain = info.brows > 0 ? (double)b_nnz / (double)info.brows : 0.0;
+  ReadSample rs;
+  if (!table && family() == 0 && a_nnz > 32768 && plain * (double)a_nnz < 1.25 * (double)nnz)
+    rs = ReadSample{A.col, B.rpt, a_nnz, 1024 * std::min(n / 1024 + (n % 1024 > 0), 16),
+                    &ctr->read_sum};
+  if ((e = launch_num_hist(crpt, n, lim, ctr->num_counts, rs, s)) != cudaSuccess)
+    return cuda_fail(e);
   ++launches;
   if ((st = fetch_counters())) return st;
   b_sorted = opts.assume_sorted || !(h.flags & B_UNSORTED);
   num_counts_ready = true;
-  intprod = (int64_t)h.total_ip;  // 0 where the row walk was skipped: B's mean row then
-  if (intprod > 0 && a_nnz > 0) info.mean_b = (double)intprod / (double)a_nnz;
-  else if (info.brows > 0) info.mean_b = (double)b_nnz / (double)info.brows;
+  const double read = rs.samples ? (double)h.read_sum / (double)rs.samples : 0.0;
+  const double each = read > 1.5 * plain ? read : plain;
+  products = h.total_ip ? (double)h.total_ip : each * (double)a_nnz;
+  if (a_nnz > 0) info.mean_b = products / (double)a_nnz;
   if ((st = build_programs()) == NSPB_ERR_ALLOC) drop_runs();
   else if (st) return st;
   if (use_runs) {
@@ -854,7 +867,7 @@ int nspb_spgemm_numeric(const nspb_csr_in *A, const nspb_csr_in *B, nspb_csr_out
   if (C->nnz < 0 || C->nnz > INT32_MAX) return NSPB_ERR_INVALID;
   if ((C->col || C->val) && (!C->col || !C->val)) return NSPB_ERR_INVALID;
   if (C->col && C->capacity < C->nnz) return NSPB_ERR_CAPACITY;
-  if ((st = call.prepare_numeric(C->rowptr))) return st;
+  if ((st = call.prepare_numeric(C->rowptr, C->nnz))) return st;
   call.h.total_nnz = C->nnz;
   bool own = false;
   if (!C->col) {

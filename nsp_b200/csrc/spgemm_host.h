@@ -27,7 +27,7 @@ struct DevCounters {
   float max_row_err;
   int max_comp_deg;  // compensated mode: largest A-row degree of a pair row
   int long_rows;     // rows listed for the block-per-row intermediate-product count
-  int pad;
+  int read_sum;      // entries of the B rows sampled (ReadSample)
   int ticket[32];    // row tickets of the block-per-row launches (symbolic
                      // bin b at b, numeric bin b at 16 + b; the runs at 30,
                      // 31, the bunches at 28, 29)
@@ -81,6 +81,9 @@ struct Call {
   bool b_sorted = true;
   bool num_counts_ready = false;
   int64_t intprod = 0;
+  // intermediate products for the choice of kernels: counted, or (a two-call
+  // numeric step that did not count them) estimated
+  double products = 0.0;
   int launches = 0;
   // Caller-supplied scratch and host staging (set by nspb_spgemm_noalloc);
   // when null the pool and the pinned per-thread stage are used.
@@ -149,7 +152,8 @@ struct Call {
     const int k = family();
     if (k == 2 || k == 3) return true;
     if (k != 0) return false;
-    return h.total_nnz > 0 && (double)intprod >= 1.5 * (double)h.total_nnz;
+    if (two_calls && !use_runs) return false;  // as before the products were counted there
+    return h.total_nnz > 0 && products >= 1.5 * (double)h.total_nnz;
   }
   // B rows whose loads the staged walk issues ahead: bits 8.. of row_kernel (0 = 4)
   // Rows a group takes in a run on the entry-map path (row templates): bits
@@ -164,14 +168,15 @@ struct Call {
   // Numeric bins up to kNumLong by sorting the products (numflat.cu): the rest
   // of the automatic choice, rows whose products are mostly entries of C of
   // their own. Their lists hold a quarter more products than entries; rows with
-  // more go to the hash kernels afterwards. A two-call numeric step, which has
-  // not counted the products, takes A's entries times B's mean row for them
-  // (both calls, power-law 37635 A*A, 12 entries a row: 695 -> 526 us).
+  // more go to the hash kernels afterwards. A two-call numeric step takes them
+  // up to 1.25 products an entry (both calls, power-law 37635 A*A, 12 entries a
+  // row: 695 -> 526 us), and the hash kernels, not the staged walk, for other
+  // rows that are in no run (14^3 27-point grid of 3 unknowns a node, the
+  // numeric kernels: 524 us, staged 842).
   bool use_flat() const {
-    if (family() != 0 || opts.num_table_shift != 0) return false;
-    if (intprod > 0) return !use_staged();
-    return info.brows > 0 && h.total_nnz > 0 &&
-           (double)a_nnz * (double)b_nnz < 1.25 * (double)h.total_nnz * (double)info.brows;
+    if (family() != 0 || opts.num_table_shift != 0 || !(products > 0.0)) return false;
+    if (!two_calls || use_runs) return !use_staged();
+    return products < 1.25 * (double)h.total_nnz;
   }
   int rg_depth() const {
     const int d = (opts.row_kernel >> 8) & 0xff;
@@ -194,7 +199,7 @@ struct Call {
   cudaError_t order_block_bins(const int *key, int kind, const int *counts, int first, int end,
                                const BinOffsets &off);
   int symbolic(int *crpt, int64_t *nnz_out);
-  int prepare_numeric(const int *crpt);
+  int prepare_numeric(const int *crpt, int64_t nnz);
   int numeric(const int *crpt, int *ccol, double *cval);
   int finish(nspb_stats *stats);
   ~Call();

@@ -1,0 +1,56 @@
+"""Which kernels a product takes, on both sides of the lines: lists or hash kernels by
+products an entry, a two-call numeric step whose A reads B's long rows above all, and rows
+of more products than runs hold. Values against the oracle; the search for runs by the
+launches of a call that is told to search (row_kernel 8)."""
+import numpy as np
+import pytest
+
+import nsp_b200 as nb
+import oracle
+from nsp_b200.csr import HostCSR
+
+from conftest import assert_bitwise, assert_same_structure
+from test_run_search_gpu import RUNS, launches
+
+pytestmark = pytest.mark.gpu
+
+
+def check(A, B, precision="fp64"):
+    f = lambda h: HostCSR(h.nrows, h.ncols, h.rowptr, h.col, h.val.astype(np.float32))  # noqa: E731
+    dA, dB = (A, B) if precision == "fp64" else (f(A), f(B))
+    dA, dB = dA.to_device(), dB.to_device()
+    rp, col, val = oracle.spgemm(A, B)
+    bound = oracle.absbound(A, B, rp, col)
+    one, st = nb.spgemm(dA, dB, precision=precision, return_stats=True)
+    rp2, nnz = nb.spgemm_symbolic(dA, dB)
+    two = nb.spgemm_numeric(dA, dB, rp2, nnz, precision=precision)
+    short = np.repeat(np.diff(rp) <= 512, np.diff(rp))
+    tol = 1e-10 if precision == "fp32c" else 2 * int(np.diff(A.rowptr).max()) * 2.0**-53
+    for C in (one, two):
+        C = C.to_host()
+        assert_same_structure(C.rowptr, C.col, rp, col)
+        assert np.all(np.abs(C.val - val) <= tol * bound)
+        if precision != "fp32c":
+            assert_bitwise(C.val[short], val[short])
+    return st
+
+
+def values(h):
+    h.val[:] = h.val.astype(np.float32)
+    return h
+
+
+@pytest.mark.parametrize("per_row", [1, 10, 40])
+@pytest.mark.parametrize("n", [900, 5000, 20_000])
+def test_a_reads_the_long_rows(cuda, n, per_row):
+    """400 B rows of 60 entries of 600 columns among 20,000 of one entry."""
+    rng = np.random.default_rng(n + per_row)
+    k, hub, m = 20_000, 400, 5000
+    rows = [np.sort(rng.choice(600, 60, replace=False)) for _ in range(hub)]
+    rows += [rng.integers(0, m, 1) for _ in range(k - hub)]
+    rp = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    B = HostCSR(k, m, rp, np.concatenate(rows).astype(np.int32), rng.uniform(-1, 1, rp[-1]))
+    col = np.concatenate([np.sort(rng.choice(hub, per_row, replace=False)) for _ in range(n)])
+    A = HostCSR(n, k, np.arange(0, n * per_row + 1, per_row, dtype=np.int32), col.astype(np.int32),
+                rng.uniform(-1, 1, n * per_row))
+    check(A, B)
