@@ -628,7 +628,14 @@ int Call::numeric(const int *crpt, int *ccol, double *cval) {
     // rows of at most 16 entries and few products on average: row groups of 8
     // lanes (300,000 rows of 4 products 93 us, from flat lists 161; 1 M of 9 380
     // and 526; the short rows of a power-law 300,000^2 of mean 6 170 and 126)
-    if (b < kNumLong && flat && !(b == 0 && lanes == 8 && few)) {
+    // Rows of up to 512 entries are ahead in their hash kernels from about 1.25
+    // products an entry on: lists and hash kernels, 20 M products, d entries a
+    // row of A and B, at 1.29, 1.39 and 1.48 products an entry: d = 12 579 and
+    // 557, 566 and 507, 570 and 498 us, d = 16 568 and 508, 568 and 470, 578 and
+    // 460, d = 20 620 and 650, 618 and 610, 652 and 615; d = 60, rows of 2400 to
+    // 2800 entries, 729 and 815, 733 and 794, 728 and 758.
+    if (b < kNumLong && flat && !(b == 0 && lanes == 8 && few) &&
+        (b >= kNumGroupBins || products < 1.25 * (double)h.total_nnz)) {
       const int o = over_bin(b);
       int *over = row_nz + over_at(o);
       e = comp ? launch_numeric_comp_flat(b, b_sorted, t32, crpt, ccol, cval, rows, c, nmax,

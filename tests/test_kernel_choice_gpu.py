@@ -40,6 +40,18 @@ def values(h):
     return h
 
 
+# d * d products a row over m columns
+@pytest.mark.parametrize("precision", ["fp64", "fp32w", "fp32c"])
+@pytest.mark.parametrize("x", [0.40, 0.46, 0.54, 0.70, 0.85])  # 1.21 to 1.48 products an entry
+@pytest.mark.parametrize("d", [4, 16, 24, 34])
+def test_products_an_entry(cuda, d, x, precision):
+    m = int(d * d / x)
+    A = values(nb.gen.random(700, 900, d, d, seed=1))
+    B = values(nb.gen.random(900, max(m, d), d, d, seed=2))
+    st = check(A, B, precision)
+    assert 1.1 < st["intprod"] / st["nnz"] < 1.6
+
+
 @pytest.mark.parametrize("per_row", [1, 10, 40])
 @pytest.mark.parametrize("n", [900, 5000, 20_000])
 def test_a_reads_the_long_rows(cuda, n, per_row):
