@@ -273,19 +273,23 @@ static BinOffsets offsets_of(const int *counts, int nb, int *nonempty, int *tota
 // 64 x 50 x 50 (7.6 M) 249 vs 314, 32^3 (1.5 M) 222 vs 170.
 // The symbolic and the numeric step in calls of their own (two_calls) search
 // twice, and need more: 14 million where B's rows are shorter than 8, 26 million
-// up to 16 if A's have at most 64 entries, 32 million otherwise. Both calls, runs against what came before
+// up to 16 if A's have at most 64 entries, 40 million otherwise. Both calls, runs against what came before
 // them: A P of 44^3 (9.8 M) 585 vs 460, of 52^3 (16.6 M) 649 vs 672; 7-point
 // 12.5 M 515 vs 497, 17.9 M 605 vs 646; R (A P) of 80^3 873 vs 818, 15-point
-// 26.6 M 539 vs 657; 27-point 31 M 566 vs 523, 43 M 608 vs 686.
+// 26.6 M 539 vs 657; 27-point 31 M 566 vs 523, 43 M 608 vs 686, 7-point 30^3 of
+// 3 unknowns a node (34 M) 738 vs 654.
 bool Call::runs_wanted() const {
   if (!allow_runs || family() != 0 || (opts.row_kernel & kNoRowTemplates)) return false;
   if (n < 2 * kRunMin || a_nnz > (int64_t)kRunMaxA * n || (table && !info.bdel)) return false;
   if ((opts.row_kernel & 0xff) == 8) return true;
   if (info.brows <= 0) return false;
   const double mean = (double)b_nnz / (double)info.brows;
+  // rows of far more products than a run may have (14^3 27-point grid of 3
+  // unknowns a node, both calls: 945 us, with the search 1010)
+  if (!table && mean * (double)a_nnz > 1.5 * kRunMaxIp * (double)n) return false;
   const double least = mean < 8.0 ? (two_calls ? 14e6 : 8e6)
                        : !two_calls ? 24e6
-                       : mean < 16.0 && a_nnz <= 64LL * n ? 26e6 : 32e6;
+                       : mean < 16.0 && a_nnz <= 64LL * n ? 26e6 : 40e6;
   return (double)a_nnz * mean >= least;
 }
 

@@ -66,3 +66,25 @@ def test_a_reads_the_long_rows(cuda, n, per_row):
     A = HostCSR(n, k, np.arange(0, n * per_row + 1, per_row, dtype=np.int32), col.astype(np.int32),
                 rng.uniform(-1, 1, n * per_row))
     check(A, B)
+
+
+def unknowns(H, d, rng):
+    """A grid of d unknowns a node."""
+    r, c = np.repeat(np.arange(H.nrows), np.diff(H.rowptr)), H.col.astype(np.int64)
+    a = np.arange(d)
+    cols = (c[:, None] * d + a).reshape(-1)  # one row of each node
+    lens = np.repeat(np.diff(H.rowptr) * d, d)
+    starts = H.rowptr[:-1] * d
+    col = np.concatenate([cols[s:s + n] for s, n in zip(np.repeat(starts, d), lens)])
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    return HostCSR(H.nrows * d, H.ncols * d, rp, col.astype(np.int32), rng.uniform(-1, 1, rp[-1]))
+
+
+def test_rows_of_too_many_products(cuda):
+    """27-point grid of 3 unknowns a node: rows of 81 entries and 6561 products."""
+    X = unknowns(nb.gen.stencil(14, npts=27), 3, np.random.default_rng(1))
+    d = X.to_device()
+    for two in (False, True):
+        auto, told = launches(d, d, 0, two), launches(d, d, RUNS, two)
+        assert all(x != y for x, y in zip(auto, told)), (auto, told)
+    check(X, X)
