@@ -29,8 +29,8 @@ NSPB_HD bool run_step_fits(int step, int rows) { return rows == 1 || step < kRun
 
 // Whether a block of k_num_run stops because a wait has run out. A look-up warp
 // or a lane may find that out at any moment, and a warp that stopped alone
-// would leave the others at their next barrier for good: every warp's view of
-// the flag goes into one vote at a barrier, `any`, and all act on its result.
+// would leave the others at their next barrier for good: the views of the flag
+// become one answer at a barrier, `any`, and all act on it.
 template <typename Lost, typename Any>
 NSPB_HD bool run_gives_up(Lost &&lost, Any &&any) {
   return any(lost());
