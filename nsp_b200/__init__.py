@@ -22,7 +22,7 @@ from .csr import DeviceCSR, HostCSR, adopt
 __all__ = ["spgemm", "spgemm_symbolic", "spgemm_numeric", "intprod", "nsp_spgemm_kernel_hash",
            "nsparseMGPU_version1", "DeviceCSR", "HostCSR", "gen", "NspbError", "lib",
            "make_opts", "stats_dict", "matio", "transpose", "sa_prolongator", "galerkin", "Plan",
-           "autotune", "spgemm_host"]
+           "autotune", "spgemm_host", "trim"]
 
 
 def _stream_ptr(stream):
@@ -106,6 +106,13 @@ def spgemm(A: DeviceCSR, B: DeviceCSR, precision: str = "fp64", out: DeviceCSR |
 def _adopt_out(c: CsrOut, vdtype="float64") -> DeviceCSR:
     return DeviceCSR(c.nrows, c.ncols, adopt(c.rowptr, c.nrows + 1, "int32"),
                      adopt(c.col, c.nnz, "int32"), adopt(c.val, c.nnz, vdtype))
+
+
+def trim() -> None:
+    """Frees the blocks of earlier outputs that the library keeps on the current
+    device for later ones (at most a sixteenth of its memory): for a program
+    whose other allocators need that memory."""
+    check(lib.nspb_trim(), "nspb_trim")
 
 
 def transpose(A: DeviceCSR, stream=None) -> DeviceCSR:
