@@ -77,7 +77,11 @@ typedef struct {
   int64_t nnz;
   const int32_t *rowptr;
   const int32_t *col;
-  const void *val;       /* nnz values of val_type                          */
+  const void *val;       /* nnz values of val_type, of any alignment that the
+                            type has; kernels that copy in bulk read whole
+                            16-byte units, so up to 15 bytes before the first
+                            and after the last value as well (never across
+                            a page, and never used)                         */
   int32_t val_type;      /* NSPB_F64 or NSPB_F32                            */
   int32_t _pad;
 } nspb_csr_in;

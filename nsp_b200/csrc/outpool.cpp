@@ -20,10 +20,10 @@
 //    cudaFree may be called it may be: it waits by freeing a block of 512 bytes
 //    (4 us; the next one is allocated first, so that the driver does not give
 //    up and map again the memory that it takes such blocks from: a product of
-//    7 points on 149 x 131 x 97 nodes took 3.0 ms instead of 1.04). cudaDeviceSynchronize would end every capture in progress on the
-//    device, also those of other threads and relaxed ones, a plan's for
-//    instance. Where cudaFree is not allowed (a global capture), the error is
-//    cudaFree's own.
+//    7 points on 149 x 131 x 97 nodes took 3.0 ms instead of 1.04).
+//    cudaDeviceSynchronize would end every capture in progress on the device,
+//    also those of other threads and relaxed ones, a plan's for instance. Where
+//    cudaFree is not allowed (a global capture), the error is cudaFree's own.
 // The blocks kept on a device hold at most a sixteenth of its memory, only
 // while a quarter of it is free, the longest unused leave first, and all of
 // them when an allocation of the library fails, for an output, for scratch or

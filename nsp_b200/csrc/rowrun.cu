@@ -1164,9 +1164,11 @@ cudaError_t launch_bunch_counts(const RunTable &rt, int nprog, int nbunch, const
 // lie one after the other (s = 1, an odd count) their values leave by one bulk
 // copy too.
 //
-// What bounds it: two 8-byte shared-memory reads and a multiply and add per
-// product, four wavefronts for 32 products, against about 22 and a barrier a
-// step for the entry-map kernel's read-modify-write of a value slot.
+// What bounds it: shared-memory wavefronts (L1 data pipe 74% on the 27-point
+// 80^3 stencil) and issue. Two 8-byte reads a product are four wavefronts for
+// 32 products; the whole kernel takes 8.8, with the program words, the sums and
+// columns written out, and the idle lanes of partial row groups. The entry-map
+// kernel takes 16.5, a read-modify-write of a value slot a product.
 constexpr int kCopyWait = 1 << 20;  // polls before a wait gives up
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
