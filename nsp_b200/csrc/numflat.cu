@@ -14,16 +14,19 @@
 // that order, so a sum is the sequential one, bit for bit, also in rows of
 // more than 512 entries, which the hash kernels add in any order.
 //
-// Bound: instruction issue (64% of the slots) and shared-memory wavefronts
-// (60% of the data pipe), at 57% occupancy by registers; DRAM is at 10%. A
+// Bound: instruction issue (62% of the slots) and shared-memory wavefronts
+// (61% of the data pipe), at 58% occupancy by registers; DRAM is at 10%. A
 // block a row keeps the rows' latencies apart; four warps and five products a
 // thread for 257..512 entries (259 us): with two warps and ten products the
 // unrolled code no longer fits the instruction cache (377 us), with eight warps
-// and three products every warp's work for the row as a whole weighs more (343). Measured on 100003 x 80021 x 120011 with
-// 4..32 entries a row (rows of 257..512 entries, 48800 of them): hash table,
-// compaction and bucket sort 694 us; products in wide buckets with a rank 322
-// us; bitmaps 259 us. All rows of that product 1160 -> 490 us; of 20 such
-// products of 1000..40000 rows in one call 4370 -> 2090 us.
+// and three products every warp's work for the row as a whole weighs more (343).
+// Measured on 100003 x 80021 x 120011 with 4..32 entries a row (rows of 257..512
+// entries, 48800 of them): hash table, compaction and bucket sort 694 us;
+// products in wide buckets with a rank 322 us; bitmaps 259 us. All rows of that
+// product 1160 -> 490 us; of 20 such products of 1000..40000 rows in one call
+// 4370 -> 2090 us. Where C's row is one row of B, in order already (a diagonal
+// times B), nothing is sorted: 27-point 64^3 rows scaled, in two calls, 480 -> 389
+// us, the columns of a stencil crowd the narrow buckets.
 #include "flat.cuh"
 #include "internal.h"
 #include "launch_util.h"
@@ -155,7 +158,7 @@ __global__ void __launch_bounds__(FlatCfg<W, K>::TH *FlatCfg<W, K>::ROWS, FlatCf
         col[i] = __ldg(op.bcol + j);
         val[i].set(ft.a[t], __ldg(op.bval + j));
       }
-    // one B row in order is the row of C already
+    // one B row in order is the row of C already (rows of one warp)
     bool copy = false;
     if constexpr (W == 1) {
       if (ne == 1) {
