@@ -249,8 +249,7 @@ cudaError_t launch_scan(const int *row_nz, int n, int *crpt, long long *total,
 // the B rows that some of A's entries read (samples: 0, or whole blocks of 1024
 // threads of the n rows, 16 at most).
 struct ReadSample {
-  const int *acol = nullptr, *brpt = nullptr;
-  int64_t a_nnz = 0;
+  const int *arpt = nullptr, *acol = nullptr, *brpt = nullptr;
   int samples = 0;
   int *sum = nullptr;  // zeroed
 };

@@ -697,9 +697,13 @@ __global__ void __launch_bounds__(1024)
   }
   if (i < rs.samples) {  // whole blocks
     const unsigned r = ((unsigned)i * 0x9e3779b1u ^ (unsigned)i >> 7) * 0x85ebca6bu >> 16;
-    const unsigned long long at = ((unsigned long long)i << 16 | r) * (unsigned long long)rs.a_nnz;
-    const int k = __ldg(rs.acol + (at / (unsigned)rs.samples >> 16));
-    const int len = min(__ldg(rs.brpt + k + 1) - __ldg(rs.brpt + k), 0xffff);
+    const int a0 = __ldg(rs.arpt), cnt = __ldg(rs.arpt + n) - a0;
+    int len = 0;
+    if (cnt > 0) {
+      const unsigned long long at = ((unsigned long long)i << 16 | r) * (unsigned)cnt;
+      const int k = __ldg(rs.acol + a0 + (int)(at / (unsigned)rs.samples >> 16));
+      len = min(__ldg(rs.brpt + k + 1) - __ldg(rs.brpt + k), 0xffff);
+    }
     const int sum = __reduce_add_sync(0xffffffffu, len);
     if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&s_sum, sum);
   }

@@ -721,7 +721,7 @@ int Call::prepare_numeric(const int *crpt, int64_t nnz) {
   const double plain = info.brows > 0 ? (double)b_nnz / (double)info.brows : 0.0;
   ReadSample rs;
   if (!table && family() == 0 && a_nnz > 32768 && plain * (double)a_nnz < 1.25 * (double)nnz)
-    rs = ReadSample{A.col, B.rpt, a_nnz, 1024 * std::min(n / 1024 + (n % 1024 > 0), 16),
+    rs = ReadSample{A.rpt, A.col, B.rpt, 1024 * std::min(n / 1024 + (n % 1024 > 0), 16),
                     &ctr->read_sum};
   if ((e = launch_num_hist(crpt, n, lim, ctr->num_counts, rs, s)) != cudaSuccess)
     return cuda_fail(e);
